@@ -1,73 +1,35 @@
 // gx_fast64.cuh -- the FP64 force in instructions the FP64 pipe can afford.
 //
-// On this part the FP64 pipe retires one warp instruction per ~64 cycles of a
-// sub-partition, and the library forms of the special operations are long
+// The FP64 unit takes one warp instruction per 19 cycles of an SM (76 of a
+// sub-partition), and the library forms of the special operations are long
 // sequences on it: sqrt and a/b cost 8 FP64-pipe instructions each, 1/x 5,
 // log ~30, pow ~84 (measured with ncu instruction counters).  The adaptive
-// DOP853 kernel, which evaluates the force 12 to 16 times a step and cannot be
-// bit-identical to gala anyway (its step control runs pow), uses the forms
-// below instead of gala's literal expressions; the fixed-step integrators and
-// the potential evaluation entry points keep gala's operation order.
+// DOP853 kernels, which evaluate the force 12 to 16 times a step and cannot be
+// bit-identical to gala anyway (their step control runs pow), use the forms
+// below instead of gala's literal expressions:
 //
-//   * sqrt and 1/x from an FP32 seed (rsqrtf / __frcp_rn of the double rounded
-//     to 23 mantissa bits, built with integer operations: no F2F conversion,
-//     which also runs on the FP64 pipe) and two Newton steps: 5 and 4 FP64
-//     instructions, within about an ulp (the seed's relative error ~3e-7 is
-//     cubed or squared twice); outside the FP32 normal range the library
-//     operations are used;
+//   * sqrt, 1/x and ln run on the integer pipe (gx_ipipe.cuh): none of them
+//     costs an FP64-pipe instruction in its usual range.  With the FP32-seeded
+//     Newton forms that stood here before (5, 4 and 14 FP64 instructions) an MW
+//     composite right-hand side took 106 of them; now 47 (DOP853 of 20,011 MW
+//     orbits x 1 Gyr: 232.9 -> 180.3 ms);
 //   * every a/b becomes a * (1/b) and products and sums are fused (fma);
 //   * gala's formulas are rearranged algebraically where that removes an
-//     operation (the NFW factor v_h^2 / u^3 / r_s^2 is G m / r^3, etc.);
-//   * ln is table-driven (log_f below, ~14 instructions instead of ~30).
+//     operation (the NFW factor v_h^2 / u^3 / r_s^2 is G m / r^3, etc.).
 // The results differ from gala's expressions by a few ulp per evaluation; the
 // integrated orbits are checked against the oracle at 1e-12 relative.
 #pragma once
 
 #include "gx_device.cuh"
+#include "gx_ipipe.cuh"
 #include "gx_log_table.cuh"
 
 namespace gx {
 namespace fast {
 
-// FP32 approximation (23 mantissa bits, truncated, sign kept) of x whose high
-// word is hi; valid when the exponent is in the FP32 normal range.
-__device__ __forceinline__ float f32_of(unsigned hi, unsigned lo) {
-    return __uint_as_float((hi & 0x80000000u) | ((((hi & 0x7fffffffu) - (896u << 20)) << 3) | (lo >> 29)));
-}
-// The double with the value of the FP32 number of bits fb (normal, any sign);
-// *half receives half of it.
-__device__ __forceinline__ double f64_of(unsigned fb, double *half) {
-    const int hi = (int)((fb & 0x80000000u) | ((((fb >> 23) & 0xffu) + 896u) << 20) | ((fb >> 3) & 0xfffffu));
-    const int lo = (int)(fb << 29);
-    if (half) *half = __hiloint2double(hi - (1 << 20), lo);
-    return __hiloint2double(hi, lo);
-}
-// |exponent| small enough that x, 1/x and 1/sqrt(x) are FP32 normal numbers
-__device__ __forceinline__ bool f32_safe(unsigned hi) {
-    const unsigned e = (hi >> 20) & 0x7ffu;
-    return e >= 1023u - 120u && e <= 1023u + 120u;
-}
-
-// sqrt(u), u >= 0: Heron steps r += (u - r^2) / (2 sqrt(u)) with the slope
-// taken from the seed.
-__device__ __forceinline__ double sqrt_f(double u) {
-    const unsigned hi = (unsigned)__double2hiint(u), lo = (unsigned)__double2loint(u);
-    if (!f32_safe(hi) || (int)hi < 0) return sqrt(u);
-    double h;
-    const double y = f64_of(__float_as_uint(rsqrtf(f32_of(hi, lo))), &h);
-    double r = u * y;
-    r = fma(fma(-r, r, u), h, r);
-    return fma(fma(-r, r, u), h, r);
-}
-
-// 1/x: Newton steps y += y (1 - x y).
-__device__ __forceinline__ double rcp_f(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    if (!f32_safe(hi)) return 1.0 / x;
-    double y = f64_of(__float_as_uint(__frcp_rn(f32_of(hi, lo))), nullptr);
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
-}
+// sqrt(u) and 1/x within 0.51 ulp, on the integer pipe.
+__device__ __forceinline__ double sqrt_f(double u) { return ip::sqrt_n(u); }
+__device__ __forceinline__ double rcp_f(double x) { return ip::rcp_n(x); }
 
 // ln x, Tang's table-driven method (P. T. P. Tang, ACM TOMS 16, 1990): x = 2^k m
 // with m in [1, 2), c_j = 1 + j/64 the nearest table point (j = 0..64), f = m - c_j
@@ -75,9 +37,12 @@ __device__ __forceinline__ double rcp_f(double x) {
 // with |r| <= 1/128 and ln(1 + r) from its Taylor series through r^9 (truncation
 // below 2^-60 relative).  ln c_j and ln 2 come in high and low parts
 // (gx_log_table.cuh, from 60-digit arithmetic).  About an ulp; 14 FP64-pipe
-// instructions against ~30 for the library log.  Zero, negative, subnormal,
-// infinite and NaN arguments go to the library.
+// instructions against ~30 for the library log.  It serves arguments below
+// 1 + 2^-6, where the integer form's fixed-point sum would lose relative
+// accuracy; zero, negative, subnormal, infinite and NaN arguments go to the
+// library.
 __device__ __forceinline__ double log_f(double x) {
+    if (ip::ln_range(x)) return ip::ln_n(x);
     const int hi = __double2hiint(x), lo = __double2loint(x);
     if (hi < 0x00100000 || hi >= 0x7ff00000) return log(x);
     const int k = (hi >> 20) - 1023;
