@@ -15,13 +15,20 @@
 // src/gala/potential/potential/builtin/builtin_potentials.cpp); the FP64
 // translation units are compiled with -fmad=false so that no multiply-add is
 // contracted, which makes the results operation-for-operation those of gala's
-// C code built without contraction.
+// C code built without contraction.  The square roots and quotients come from
+// the integer pipe (gx_ipipe.cuh: correctly rounded, so the same bits as the FP64
+// instructions they replace, 8 FP64-pipe instructions each) and so does ln (within
+// 0.65 ulp, the library's is within 1); products of parameters are formed once on
+// the host, and the radius once per point for all components that are neither
+// shifted nor rotated.  An MW-composite gradient takes 51 FP64-pipe instructions
+// that way instead of about 200.
 #pragma once
 
 #include <cstdint>
 #include <cuda_runtime.h>
 
 #include "../../include/gala_gb300.h"
+#include "gx_ipipe.cuh"
 
 namespace gx {
 
@@ -32,18 +39,19 @@ struct DevComp {
     int32_t inl;      // 1: parameters are in DevPot::p; 0: in pdev (SCF)
     double q0[3];
     double R[9];
-    // Constants derived from the parameters on the host (for the forms of
-    // gx_fast64.cuh): dc[0] = G m; Plummer, Miyamoto-Nagai: dc[1] = b^2;
-    // NFW: dc[1] = 1 / r_s, dc[2..4] = 1 / a^2, 1 / b^2, 1 / c^2 (1 where the
-    // shape has no such axis).
-    double dc[5];
+    // Constants derived from the parameters on the host, each the IEEE result of
+    // gala's own expression where gala forms it: dc[0] = G m; Plummer,
+    // Miyamoto-Nagai: dc[1] = b^2; NFW: dc[1] = 1 / r_s, dc[2..4] = 1 / a^2,
+    // 1 / b^2, 1 / c^2 (1 where the shape has no such axis), dc[5] = G m / r_s,
+    // dc[6] = r_s^2.
+    double dc[7];
 };
 
 struct DevPot {
     int32_t ncomp;
     int32_t n_inline;
     int32_t has_scf;      // selects the SCF = true instantiation on the host
-    int32_t pad;
+    int32_t regular;      // see finite_gradient below
     const double *pdev;   // device copy of the packed parameters (may be null)
     const DevComp *cdev;  // component table in device memory (more than
                           // GX_MAX_COMPONENTS components), else null
@@ -81,6 +89,20 @@ __device__ __forceinline__ double norm3_sq(const double *q) {
     return q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
 }
 
+// gala's sqrt(x), a / b and log(x).  LIBLN takes the library's ln instead of the
+// integer one (30 FP64-pipe instructions more per NFW gradient; one evaluation in
+// 300 differs in the last bit).  The Leapfrog n-body kernels ask for it, and so
+// does every potential value: stream particles bound to a light progenitor move
+// chaotically at Leapfrog's step, so a last-bit change of the force, or of the
+// second difference of Phi that places them, moves a few of them by 1e-3 kpc.
+__device__ __forceinline__ double dsqrt(double x) { return ip::sqrt_rn(x); }
+__device__ __forceinline__ double ddiv(double a, double b) { return ip::div_rn(a, b); }
+template <bool LIBLN>
+__device__ __forceinline__ double dlog(double x) {
+    if (!LIBLN && ip::ln_range(x)) return ip::ln_n(x);
+    return log(x);
+}
+
 // Powers in the gradients.  gala calls pow(x, -1.5) (Miyamoto-Nagai) and
 // pow(r, 3.0) (Kepler).  The FP64 pow of CUDA runs an extended-precision log
 // and exp, a hundred-odd instructions on the FP64 pipe, whose rate on this part
@@ -88,8 +110,44 @@ __device__ __forceinline__ double norm3_sq(const double *q) {
 // operations (within 1.5 ulp of x^-1.5) and r r r within 1 ulp of r^3: the
 // accuracy class of pow itself, which does not round like the host's pow
 // either.  Edge values match pow: 0 -> inf, inf -> 0, NaN -> NaN.
-__device__ __forceinline__ double pow_m1p5(double x) { return 1.0 / (x * sqrt(x)); }
+__device__ __forceinline__ double pow_m1p5(double x) { return ddiv(1.0, x * dsqrt(x)); }
 __device__ __forceinline__ double cube(double r) { return r * r * r; }
+
+// x^2 + y^2 + z^2 and its root at one point, formed when a component first asks
+// for them and kept for the others at the same point (the same expressions, so
+// the same bits).
+struct Radius {
+    double s, r;
+    int have;  // 1: s, 2: s and r
+    __device__ __forceinline__ double sq(const double *q) {
+        if (have == 0) {
+            s = norm3_sq(q);
+            have = 1;
+        }
+        return s;
+    }
+    __device__ __forceinline__ double root(const double *q) {
+        if (have < 2) {
+            r = dsqrt(sq(q));
+            have = 2;
+        }
+        return r;
+    }
+};
+
+// Whether the gradient at x is finite for certain, so that gala's product of it
+// with a zero coefficient (the first sub-step of Ruth4) is zero: `regular` says
+// that every component is a closed form centred on the origin with parameters of
+// ordinary size (regular_potential in gx_host.cu), and the largest coordinate
+// lies within 2^-100 and 2^100.
+__device__ __forceinline__ bool ordinary(double v) {
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) - (923u << 20) < (200u << 20);
+}
+__device__ __forceinline__ bool finite_gradient(const DevPot &pot, const double *x) {
+    const unsigned m = 0x7fffffffu;
+    const unsigned h = max((unsigned)__double2hiint(x[0]) & m, max((unsigned)__double2hiint(x[1]) & m, (unsigned)__double2hiint(x[2]) & m));
+    return pot.regular && h - (923u << 20) < (200u << 20);
+}
 
 // Parameters of component ci as a plain pointer: inline ones are read from the
 // kernel-parameter copy, SCF blocks from global memory.
@@ -99,115 +157,104 @@ __device__ __forceinline__ double cube(double r) { return r * r * r; }
 // plummer_value :292-300, miyamotonagai_value :1287-1296, sphericalnfw_value
 // :819-833, flattenednfw_value :925-942, triaxialnfw_value :1028-1049).
 template <bool SCF, typename PV>
-__device__ __forceinline__ double comp_value(const PV &pot, int ci, const double *q) {
-    const int type = pot.c[ci].type;
+__device__ __forceinline__ double comp_value(const PV &pot, int ci, const double *q, Radius &R) {
+    const DevComp &C = pot.c[ci];
 #define P(k) GX_PARAM(pot, ci, k)
-    switch (type) {
+    double u;
+    switch (C.type) {
     case GX_POT_NULL:
         return 0.;
     case GX_POT_KEPLER:
-        return -P(0) * P(1) / sqrt(norm3_sq(q));
-    case GX_POT_HERNQUIST: {
-        const double r = sqrt(norm3_sq(q));
-        return -P(0) * P(1) / (r + P(2));
-    }
-    case GX_POT_PLUMMER: {
-        const double r2 = norm3_sq(q);
-        return -P(0) * P(1) / sqrt(r2 + P(2) * P(2));
-    }
+        return ddiv(-C.dc[0], R.root(q));
+    case GX_POT_HERNQUIST:
+        return ddiv(-C.dc[0], R.root(q) + P(2));
+    case GX_POT_PLUMMER:
+        return ddiv(-C.dc[0], dsqrt(R.sq(q) + C.dc[1]));
     case GX_POT_MIYAMOTONAGAI: {
-        const double zd = (P(2) + sqrt(q[2] * q[2] + P(3) * P(3)));
-        return -P(0) * P(1) / sqrt(q[0] * q[0] + q[1] * q[1] + zd * zd);
+        const double zd = (P(2) + dsqrt(q[2] * q[2] + C.dc[1]));
+        return ddiv(-C.dc[0], dsqrt(q[0] * q[0] + q[1] * q[1] + zd * zd));
     }
-    case GX_POT_SPHERICALNFW: {
-        const double v_h2 = -P(0) * P(1) / P(2);
-        const double u = sqrt(norm3_sq(q)) / P(2);
-        if (u == 0) return v_h2;
-        return v_h2 * log(1 + u) / u;
-    }
-    case GX_POT_FLATTENEDNFW: {
-        const double v_h2 = -P(0) * P(1) / P(2);
-        const double u = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] / (P(5) * P(5))) / P(2);
-        if (u == 0) return v_h2;
-        return v_h2 * log(1 + u) / u;
-    }
-    case GX_POT_TRIAXIALNFW: {
-        const double v_h2 = -P(0) * P(1) / P(2);
-        const double u = sqrt(q[0] * q[0] / (P(3) * P(3)) + q[1] * q[1] / (P(4) * P(4)) +
-                              q[2] * q[2] / (P(5) * P(5))) / P(2);
-        if (u == 0) return v_h2;
-        return v_h2 * log(1 + u) / u;
-    }
+    case GX_POT_SPHERICALNFW:
+        u = ddiv(R.root(q), P(2));
+        break;
+    case GX_POT_FLATTENEDNFW:
+        u = ddiv(dsqrt(q[0] * q[0] + q[1] * q[1] + ddiv(q[2] * q[2], P(5) * P(5))), P(2));
+        break;
+    case GX_POT_TRIAXIALNFW:
+        u = ddiv(dsqrt(ddiv(q[0] * q[0], P(3) * P(3)) + ddiv(q[1] * q[1], P(4) * P(4)) + ddiv(q[2] * q[2], P(5) * P(5))), P(2));
+        break;
     case GX_POT_SCF:
-        if constexpr (SCF) return scf_value_dev(pot.pdev + pot.c[ci].poff, q);
+        if constexpr (SCF) return scf_value_dev(pot.pdev + C.poff, q);
         return __longlong_as_double(0x7ff8000000000000LL);
     default:
         return __longlong_as_double(0x7ff8000000000000LL);
     }
+    // the three NFW shapes (v_h^2 = -G m / r_s)
+    if (u == 0) return -C.dc[5];
+    return ddiv(-C.dc[5] * log(1 + u), u);
 #undef P
 }
 
 // Gradient of one component, accumulated into g (kepler :66-76, hernquist
 // :221-233, plummer :302-314, miyamotonagai :1298-1312, sphericalnfw :835-850,
 // flattenednfw :944-962, triaxialnfw :1051-1072).
-template <bool SCF, typename PV>
-__device__ __forceinline__ void comp_gradient(const PV &pot, int ci, const double *q, double *g) {
-    const int type = pot.c[ci].type;
+template <bool SCF, bool LIBLN, typename PV>
+__device__ __forceinline__ void comp_gradient(const PV &pot, int ci, const double *q, double *g, Radius &R) {
+    const DevComp &C = pot.c[ci];
 #define P(k) GX_PARAM(pot, ci, k)
-    double fac;
-    switch (type) {
+    double fac, u;
+    switch (C.type) {
     case GX_POT_NULL:
         return;
     case GX_POT_KEPLER:
-        fac = P(0) * P(1) / cube(sqrt(norm3_sq(q)));
+        fac = ddiv(C.dc[0], cube(R.root(q)));
         break;
     case GX_POT_HERNQUIST: {
-        const double r = sqrt(norm3_sq(q));
-        fac = P(0) * P(1) / ((r + P(2)) * (r + P(2)) * r);
+        const double r = R.root(q);
+        fac = ddiv(C.dc[0], (r + P(2)) * (r + P(2)) * r);
         break;
     }
     case GX_POT_PLUMMER: {
-        const double R2b = norm3_sq(q) + P(2) * P(2);
-        fac = P(0) * P(1) / sqrt(R2b) / R2b;
+        const double R2b = R.sq(q) + C.dc[1];
+        fac = ddiv(ddiv(C.dc[0], dsqrt(R2b)), R2b);
         break;
     }
     case GX_POT_MIYAMOTONAGAI: {
-        const double sqrtz = sqrt(q[2] * q[2] + P(3) * P(3));
+        const double sqrtz = dsqrt(q[2] * q[2] + C.dc[1]);
         const double zd = P(2) + sqrtz;
-        fac = P(0) * P(1) * pow_m1p5(q[0] * q[0] + q[1] * q[1] + zd * zd);
+        fac = C.dc[0] * pow_m1p5(q[0] * q[0] + q[1] * q[1] + zd * zd);
         g[0] = g[0] + fac * q[0];
         g[1] = g[1] + fac * q[1];
-        g[2] = g[2] + fac * q[2] * (1. + P(2) / sqrtz);
+        g[2] = g[2] + fac * q[2] * (1. + ddiv(P(2), sqrtz));
         return;
     }
-    case GX_POT_SPHERICALNFW: {
-        const double v_h2 = P(0) * P(1) / P(2);
-        const double u = sqrt(norm3_sq(q)) / P(2);
-        fac = v_h2 / (u * u * u) / (P(2) * P(2)) * (log(1 + u) - u / (1 + u));
-        break;
-    }
-    case GX_POT_FLATTENEDNFW: {
-        const double v_h2 = P(0) * P(1) / P(2);
-        const double u = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] / (P(5) * P(5))) / P(2);
-        fac = v_h2 / (u * u * u) / (P(2) * P(2)) * (log(1 + u) - u / (1 + u));
-        g[0] = g[0] + fac * q[0];
-        g[1] = g[1] + fac * q[1];
-        g[2] = g[2] + fac * q[2] / (P(5) * P(5));
-        return;
-    }
+    case GX_POT_SPHERICALNFW:
+    case GX_POT_FLATTENEDNFW:
     case GX_POT_TRIAXIALNFW: {
-        const double v_h2 = P(0) * P(1) / P(2);
-        const double u = sqrt(q[0] * q[0] / (P(3) * P(3)) + q[1] * q[1] / (P(4) * P(4)) +
-                              q[2] * q[2] / (P(5) * P(5))) / P(2);
-        fac = v_h2 / (u * u * u) / (P(2) * P(2)) * (log(1 + u) - u / (1 + u));
-        g[0] = g[0] + fac * q[0] / (P(3) * P(3));
-        g[1] = g[1] + fac * q[1] / (P(4) * P(4));
-        g[2] = g[2] + fac * q[2] / (P(5) * P(5));
+        double m;
+        if (C.type == GX_POT_SPHERICALNFW)
+            m = R.root(q);
+        else if (C.type == GX_POT_FLATTENEDNFW)
+            m = dsqrt(q[0] * q[0] + q[1] * q[1] + ddiv(q[2] * q[2], P(5) * P(5)));
+        else
+            m = dsqrt(ddiv(q[0] * q[0], P(3) * P(3)) + ddiv(q[1] * q[1], P(4) * P(4)) + ddiv(q[2] * q[2], P(5) * P(5)));
+        u = ddiv(m, P(2));
+        const double u1 = 1 + u;
+        fac = ddiv(ddiv(C.dc[5], u * u * u), C.dc[6]) * (dlog<LIBLN>(u1) - ddiv(u, u1));
+        if (C.type == GX_POT_SPHERICALNFW) break;
+        if (C.type == GX_POT_FLATTENEDNFW) {
+            g[0] = g[0] + fac * q[0];
+            g[1] = g[1] + fac * q[1];
+        } else {
+            g[0] = g[0] + ddiv(fac * q[0], P(3) * P(3));
+            g[1] = g[1] + ddiv(fac * q[1], P(4) * P(4));
+        }
+        g[2] = g[2] + ddiv(fac * q[2], P(5) * P(5));
         return;
     }
     case GX_POT_SCF:
         if constexpr (SCF) {
-            scf_gradient_dev(pot.pdev + pot.c[ci].poff, q, g);
+            scf_gradient_dev(pot.pdev + C.poff, q, g);
             return;
         }
         fac = __longlong_as_double(0x7ff8000000000000LL);
@@ -283,13 +330,17 @@ __device__ __forceinline__ void shift_rotate(const DevComp &c, const double *q, 
 template <bool SCF, typename PV>
 __device__ __forceinline__ double potential_value_t(const PV &pot, const double *q) {
     double v = 0;
+    Radius R;
+    R.have = 0;
     for (int i = 0; i < pot.ncomp; i++) {
         if (pot.c[i].do_sr == 0) {
-            v = v + comp_value<SCF>(pot, i, q);
+            v = v + comp_value<SCF>(pot, i, q, R);
         } else {
             double qt[3];
+            Radius Rt;
+            Rt.have = 0;
             shift_rotate(pot.c[i], q, qt);
-            v = v + comp_value<SCF>(pot, i, qt);
+            v = v + comp_value<SCF>(pot, i, qt, Rt);
         }
     }
     return v;
@@ -314,17 +365,21 @@ __device__ __forceinline__ double potential_density_t(const PV &pot, const doubl
 // c_gradient at one point (cpotential.cpp:214-287): zero, accumulate each
 // component in order; shifted/rotated components go through a zeroed
 // temporary, are rotated back with R^T (apply_rotate_T, :103-134) and added.
-template <bool SCF, typename PV>
+template <bool SCF, bool LIBLN, typename PV>
 __device__ __forceinline__ void potential_gradient_t(const PV &pot, const double *q, double *g) {
     g[0] = 0.; g[1] = 0.; g[2] = 0.;
+    Radius R;
+    R.have = 0;
     for (int i = 0; i < pot.ncomp; i++) {
         if (pot.c[i].do_sr == 0) {
-            comp_gradient<SCF>(pot, i, q, g);
+            comp_gradient<SCF, LIBLN>(pot, i, q, g, R);
         } else {
             const DevComp &c = pot.c[i];
             double qt[3], gt[3] = {0., 0., 0.};
+            Radius Rt;
+            Rt.have = 0;
             shift_rotate(c, q, qt);
-            comp_gradient<SCF>(pot, i, qt, gt);
+            comp_gradient<SCF, LIBLN>(pot, i, qt, gt, Rt);
             g[0] += c.R[0] * gt[0] + c.R[3] * gt[1] + c.R[6] * gt[2];
             g[1] += c.R[1] * gt[0] + c.R[4] * gt[1] + c.R[7] * gt[2];
             g[2] += c.R[2] * gt[0] + c.R[5] * gt[1] + c.R[8] * gt[2];
@@ -344,13 +399,13 @@ __device__ __forceinline__ double potential_density(const DevPot &pot, const dou
     if (pot.cdev) return potential_density_t<SCF>(table_view(pot), q);
     return potential_density_t<SCF>(pot, q);
 }
-template <bool SCF>
+template <bool SCF, bool LIBLN = false>
 __device__ __forceinline__ void potential_gradient(const DevPot &pot, const double *q, double *g) {
     if (pot.cdev) {
-        potential_gradient_t<SCF>(table_view(pot), q, g);
+        potential_gradient_t<SCF, LIBLN>(table_view(pot), q, g);
         return;
     }
-    potential_gradient_t<SCF>(pot, q, g);
+    potential_gradient_t<SCF, LIBLN>(pot, q, g);
 }
 
 // Frame energy: static_frame_hamiltonian (builtin_frames.cpp:8-16) or
@@ -411,10 +466,10 @@ struct V6 {
     double v[6];
 };
 
-template <bool SCF>
+template <bool SCF, bool LIBLN = false>
 __device__ __noinline__ V3 gradient_call(const DevPot &pot, V3 q) {
     V3 g;
-    potential_gradient<SCF>(pot, q.v, g.v);
+    potential_gradient<SCF, LIBLN>(pot, q.v, g.v);
     return g;
 }
 

@@ -485,3 +485,26 @@ extern "C" int gx_selfcheck_fast64(const double *x, int64_t n, double *out, void
     gx::selfcheck_fast64_kernel<<<(unsigned)((n + 255) / 256), 256, 0, gx::as_stream(stream)>>>(x, n, out);
     return gx::check_launch("selfcheck_fast64");
 }
+
+namespace gx {
+__global__ void selfcheck_ipipe_kernel(const double *__restrict__ x, const double *__restrict__ y, int64_t n,
+                                       double *__restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double rs;
+    out[i] = ip::sqrt_rn(x[i]);
+    out[n + i] = ip::div_rn(x[i], y[i]);
+    out[2 * n + i] = sqrt(x[i]);
+    out[3 * n + i] = x[i] / y[i];
+    out[4 * n + i] = ip::sqrt_rsqrt_n(x[i], rs);
+    out[5 * n + i] = rs;
+}
+}  // namespace gx
+
+extern "C" int gx_selfcheck_ipipe(const double *x, const double *y, int64_t n, double *out, void *stream) {
+    GX_CHECK_ARG(n >= 0, "n < 0");
+    if (n == 0) return GX_OK;
+    GX_CHECK_ARG(x && y && out, "NULL array");
+    gx::selfcheck_ipipe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, gx::as_stream(stream)>>>(x, y, n, out);
+    return gx::check_launch("selfcheck_ipipe");
+}

@@ -168,7 +168,7 @@ __device__ __forceinline__ void potential_gradient_ft(const PV &pot, const doubl
 template <bool SCF>
 __device__ __forceinline__ void potential_gradient_f(const DevPot &pot, const double *q, double *g) {
     if (pot.cdev) {
-        potential_gradient_t<SCF>(table_view(pot), q, g);
+        potential_gradient_t<SCF, false>(table_view(pot), q, g);
         return;
     }
     potential_gradient_ft<SCF>(pot, q, g);

@@ -7,6 +7,13 @@
 // rows.  The per-orbit arithmetic is gala's, expression by expression:
 //   leapfrog  c_init_velocity / c_leapfrog_step (leapfrog.pyx:24-51,99-116)
 //   ruth4     c_ruth4_step with gala's coefficients (ruth4.pyx:24-35,65-78,98-108)
+// What bounds them is the FP64 pipe: one warp alone on a scheduler retires an
+// FP64 instruction per 64 cycles whatever it depends on.  Roots and quotients on
+// the integer pipe (gx_device.cuh), Ruth4's zero-weight gradient left out where
+// it is certainly finite, and Leapfrog's synchronised velocity formed only where
+// it is stored took 16,384 uneven orbits (100 to 2,000 steps) from 69.8 to 35.5 ms
+// and 1,024 Hernquist orbits x 1,000 stored steps from 2.37 to 1.80 ms, with the
+// same bits (ln, in NFW, within an ulp).
 #include "gx_host.h"
 #include "gx_queue.cuh"
 #include "gx_scf.cuh"
@@ -25,6 +32,27 @@ __device__ __forceinline__ void grad_impl(const DevPot &pot, const double *x, do
     g[0] = r.v[0]; g[1] = r.v[1]; g[2] = r.v[2];
 }
 #define grad(pot, x, g) grad_impl<SCF>(pot, x, g)
+
+// gala's v - g * dt / 2 from gd = g * dt: halving is exact, so the fused form
+// rounds once, as the subtraction does.
+__device__ __forceinline__ double half_kick(double v, double gd) { return fma(-0.5, gd, v); }
+
+// One Ruth4 step (c_ruth4_step).  The first sub-step has d = 0, yet gala still
+// evaluates the gradient there: a non-finite gradient (an orbit sitting on a
+// singular point) turns v into NaN through 0 * inf.  Where the gradient is finite
+// for certain (finite_gradient, and a step of ordinary size) the product is zero
+// and the evaluation is left out: a quarter of the step.
+template <bool SCF>
+__device__ __forceinline__ void ruth4_step(const DevPot &pot, const Ruth4Coef &co, double dt, bool dt_ok, double *w) {
+    double g[3];
+    for (int s = 0; s < 4; s++) {
+        if (s > 0 || !(dt_ok && finite_gradient(pot, w))) {
+            grad(pot, w, g);
+            for (int k = 0; k < 3; k++) w[3 + k] = w[3 + k] - co.d[s] * g[k] * dt;
+        }
+        for (int k = 0; k < 3; k++) w[k] = w[k] + co.c[s] * w[3 + k] * dt;
+    }
+}
 
 template <bool SAVE_ALL, bool SCF>
 __global__ void __launch_bounds__(128, 1) leapfrog_kernel(const __grid_constant__ DevPot pot, const double *__restrict__ w0, int64_t n,
@@ -46,14 +74,16 @@ __global__ void __launch_bounds__(128, 1) leapfrog_kernel(const __grid_constant_
     }
     // c_init_velocity: v_{1/2} = v - grad * dt / 2
     grad(pot, x, g);
-    for (int k = 0; k < 3; k++) vh[k] = v[k] - g[k] * dt / 2.;
+    for (int k = 0; k < 3; k++) vh[k] = half_kick(v[k], g[k] * dt);
     for (int64_t j = 1; j < ntimes; j++) {
         // c_leapfrog_step: drift, gradient, half kick (output v), full kick
         for (int k = 0; k < 3; k++) x[k] = x[k] + vh[k] * dt;
         grad(pot, x, g);
         for (int k = 0; k < 3; k++) {
-            v[k] = vh[k] - g[k] * dt / 2.;
-            vh[k] = vh[k] - g[k] * dt;
+            const double gd = g[k] * dt;
+            // v is an output only: formed where it is stored
+            if (SAVE_ALL || j == ntimes - 1) v[k] = half_kick(vh[k], gd);
+            vh[k] = vh[k] - gd;
         }
         if (SAVE_ALL) {
             for (int k = 0; k < 3; k++) {
@@ -76,24 +106,14 @@ __global__ void __launch_bounds__(128, 1) ruth4_kernel(const __grid_constant__ D
                                                     double *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double w[6], g[3];
+    double w[6];
     for (int k = 0; k < 6; k++) w[k] = w0[k * n + i];
     const double dt = t[1] - t[0];
+    const bool dt_ok = ordinary(dt);
     if (SAVE_ALL)
         for (int k = 0; k < 6; k++) out[(k * ntimes) * n + i] = w[k];
     for (int64_t j = 1; j < ntimes; j++) {
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-            // The first sub-step has d = 0, yet gala still evaluates the gradient
-            // there: a non-finite gradient (an orbit sitting on a singular point)
-            // turns v into NaN through 0 * inf.  This FP64 form keeps that
-            // evaluation so that it reproduces gala in every case.
-            grad(pot, w, g);
-            for (int k = 0; k < 3; k++) {
-                w[3 + k] = w[3 + k] - co.d[s] * g[k] * dt;
-                w[k] = w[k] + co.c[s] * w[3 + k] * dt;
-            }
-        }
+        ruth4_step<SCF>(pot, co, dt, dt_ok, w);
         if (SAVE_ALL)
             for (int k = 0; k < 6; k++) __stcs(&out[(k * ntimes + j) * n + i], w[k]);
     }
@@ -145,25 +165,19 @@ __global__ void __launch_bounds__(128, 1) batch_fp64_kernel(const __grid_constan
             if (ns > 0 && method[i] == 0) {
                 double vh[3];
                 grad(pot, w, g);
-                for (int k = 0; k < 3; k++) vh[k] = w[3 + k] - g[k] * dt / 2.;
+                for (int k = 0; k < 3; k++) vh[k] = half_kick(w[3 + k], g[k] * dt);
                 for (int64_t j = 0; j < ns; j++) {
                     for (int k = 0; k < 3; k++) w[k] = w[k] + vh[k] * dt;
                     grad(pot, w, g);
                     for (int k = 0; k < 3; k++) {
-                        w[3 + k] = vh[k] - g[k] * dt / 2.;
-                        vh[k] = vh[k] - g[k] * dt;
+                        const double gd = g[k] * dt;
+                        if (j == ns - 1) w[3 + k] = half_kick(vh[k], gd);
+                        vh[k] = vh[k] - gd;
                     }
                 }
             } else if (ns > 0) {
-                for (int64_t j = 0; j < ns; j++) {
-                    for (int s = 0; s < 4; s++) {
-                        grad(pot, w, g);
-                        for (int k = 0; k < 3; k++) {
-                            w[3 + k] = w[3 + k] - co.d[s] * g[k] * dt;
-                            w[k] = w[k] + co.c[s] * w[3 + k] * dt;
-                        }
-                    }
-                }
+                const bool dt_ok = ordinary(dt);
+                for (int64_t j = 0; j < ns; j++) ruth4_step<SCF>(pot, co, dt, dt_ok, w);
             }
             for (int k = 0; k < 6; k++) out[k * n + i] = w[k];
         }

@@ -40,8 +40,7 @@ int expected_params(int type, const double *p, int64_t avail) {
     }
 }
 
-// Host-derived constants of a component for the FP64-pipe-lean forms
-// (gx_fast64.cuh); P is the component's [G, ...] block.
+// Host-derived constants of a component (gx_device.cuh, DevComp::dc); P is the component's [G, ...] block.
 static void derived_constants(int type, const double *P, DevComp &d) {
     d.dc[0] = P[0] * P[1];
     switch (type) {
@@ -54,8 +53,34 @@ static void derived_constants(int type, const double *P, DevComp &d) {
         d.dc[2] = type == GX_POT_TRIAXIALNFW ? 1.0 / (P[3] * P[3]) : 1.0;
         d.dc[3] = type == GX_POT_TRIAXIALNFW ? 1.0 / (P[4] * P[4]) : 1.0;
         d.dc[4] = type != GX_POT_SPHERICALNFW ? 1.0 / (P[5] * P[5]) : 1.0;
+        d.dc[5] = P[0] * P[1] / P[2];
+        d.dc[6] = P[2] * P[2];
         break;
     default: break;
+    }
+}
+
+// Whether the component's gradient is finite wherever the largest coordinate lies
+// within 2^-100 and 2^100: centred on the origin, every length positive (Hernquist
+// c and Miyamoto-Nagai a may be 0, Plummer b anything) and every parameter of
+// ordinary size.  Then no intermediate of its gradient leaves the FP64 range (the
+// largest is G m / r_s / u^3 / r_s^2 with u = r / r_s >= 2^-160) and no divisor is zero.
+static bool regular_component(int type, const double *P, int do_sr) {
+    if (do_sr) return false;
+    auto small = [](double v) { return std::fabs(v) <= std::ldexp(1.0, 60); };
+    auto length = [](double v) { return v >= std::ldexp(1.0, -60) && v <= std::ldexp(1.0, 60); };
+    auto length0 = [](double v) { return v >= 0 && v <= std::ldexp(1.0, 60); };
+    if (type != GX_POT_NULL && !(small(P[0]) && small(P[1]))) return false;
+    switch (type) {
+    case GX_POT_NULL:
+    case GX_POT_KEPLER: return true;
+    case GX_POT_HERNQUIST: return length0(P[2]);
+    case GX_POT_PLUMMER: return small(P[2]);
+    case GX_POT_MIYAMOTONAGAI: return length0(P[2]) && length(P[3]);
+    case GX_POT_SPHERICALNFW: return length(P[2]);
+    case GX_POT_FLATTENEDNFW: return length(P[2]) && length(P[5]);
+    case GX_POT_TRIAXIALNFW: return length(P[2]) && length(P[3]) && length(P[4]) && length(P[5]);
+    default: return false;
     }
 }
 
@@ -105,6 +130,7 @@ int pack_potential(const gx_potential *pot, DevPot *out) {
         return GX_OK;
     }
     int ninl = 0;
+    out->regular = 1;
     for (int i = 0; i < pot->n_components; i++) {
         const gx_component &c = pot->components[i];
         int need = 0;
@@ -134,6 +160,7 @@ int pack_potential(const gx_potential *pot, DevPot *out) {
             ninl += need;
             derived_constants(c.type, pot->params + c.param_offset, d);
         }
+        if (!regular_component(c.type, pot->params + c.param_offset, d.do_sr)) out->regular = 0;
     }
     out->n_inline = ninl;
     return GX_OK;

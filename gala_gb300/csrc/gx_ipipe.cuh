@@ -187,8 +187,8 @@ __device__ __forceinline__ uint32_t rsqrt_seed(uint32_t fb) {
 __device__ __forceinline__ uint32_t top23(uint32_t hi, uint32_t lo) { return ((hi << 3) | (lo >> 29)) & 0x7fffffu; }
 // normal and not negative
 __device__ __forceinline__ bool normal_pos(uint32_t hi) { return hi - 0x00100000u < 0x7fe00000u; }
-// |x| in [2^-512, 2^512)
-__device__ __forceinline__ bool mid_range(uint32_t hi) { return (hi & 0x7fffffffu) - (511u << 20) < (1024u << 20); }
+// |x| in [2^-511, 2^511): quotients of two such numbers are normal
+__device__ __forceinline__ bool mid_range(uint32_t hi) { return (hi & 0x7fffffffu) - (512u << 20) < (1022u << 20); }
 // (e + 1) 2^52 + R with R in [2^52, 2^53]: the double of value R 2^-52 2^e, ebits = (e + 1022) << 20
 __device__ __forceinline__ double pack53(uint64_t R, uint32_t ebits) {
     return __longlong_as_double((long long)(R + ((uint64_t)ebits << 32)));

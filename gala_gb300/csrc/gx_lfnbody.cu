@@ -46,7 +46,7 @@ __device__ __forceinline__ void lf_grad(const DevPot &pot, const gx_body *__rest
     q.v[0] = x[b][0];
     q.v[1] = x[b][1];
     q.v[2] = x[b][2];
-    const V3 ge = gradient_call<SCF>(pot, q);
+    const V3 ge = gradient_call<SCF, true>(pot, q);
     g[0] = ge.v[0];
     g[1] = ge.v[1];
     g[2] = ge.v[2];
@@ -55,7 +55,7 @@ __device__ __forceinline__ void lf_grad(const DevPot &pot, const gx_body *__rest
         if (j >= nbody || j == b) continue;
         const int type = __ldg(&bod[j].type);
         if (type == GX_POT_NULL) continue;
-        const V3 f2 = body_gradient_call(type, bod[j].params, x[b][0] - x[j][0], x[b][1] - x[j][1],
+        const V3 f2 = body_gradient_call<true>(type, bod[j].params, x[b][0] - x[j][0], x[b][1] - x[j][1],
                                          x[b][2] - x[j][2]);
         g[0] += f2.v[0];
         g[1] += f2.v[1];

@@ -91,11 +91,10 @@ __device__ __forceinline__ void wide_rhs(const DevPot &pot, const DevFrame &fr, 
     for (int j = 0; j < nbody; j++) {
         const int type = __ldg(&bod[j].type);
         if (j == m || type == GX_POT_NULL) continue;
-        double f2[3];
-        body_gradient(type, bod[j].params, w.v[0] - arg[j], w.v[1] - arg[M + j], w.v[2] - arg[2 * M + j], f2);
-        k.v[3] += -f2[0];
-        k.v[4] += -f2[1];
-        k.v[5] += -f2[2];
+        const V3 f2 = body_gradient_call(type, bod[j].params, w.v[0] - arg[j], w.v[1] - arg[M + j], w.v[2] - arg[2 * M + j]);
+        k.v[3] += -f2.v[0];
+        k.v[4] += -f2.v[1];
+        k.v[5] += -f2.v[2];
     }
 #pragma unroll
     for (int c = 0; c < 6; c++) kout[c * M + m] = k.v[c];

@@ -495,9 +495,15 @@ int gx_calibrate_fma(int32_t fp64, int32_t blocks, int32_t threads, int64_t iter
 
 /* Numerics self-check of the FP64 forms the DOP853 force uses instead of the
  * library functions (no counterpart in gala): for n DEVICE doubles x, out is
- * (4, n) DEVICE doubles: the table-driven ln x, the library log(x), the
- * seeded-Newton sqrt(x) and 1/x. */
+ * (4, n) DEVICE doubles: the table-driven ln x, the library log(x), and sqrt(x)
+ * and 1/x from the integer pipe. */
 int gx_selfcheck_fast64(const double* x, int64_t n, double* out, void* stream);
+
+/* The same for the correctly rounded forms of the literal expressions: for n
+ * DEVICE doubles x and y, out is (6, n) DEVICE doubles: sqrt(x) and x / y from
+ * the integer pipe, the same two from the FP64 pipe, and sqrt(x) and
+ * 1 / sqrt(x) from the shared core (each within an ulp). */
+int gx_selfcheck_ipipe(const double* x, const double* y, int64_t n, double* out, void* stream);
 
 /* ------------------------------------------------------------------------- */
 /* Direct n-body systems and mock streams                                    */
