@@ -5,149 +5,173 @@
 // phi_nl / rho_nl / sph_grad_phi_nlm (bfe_helper.cpp:14-90), with gala's
 // coefficient packing p = [G, nmax, lmax, M, r_s, S[n][l][m], T[n][l][m]].
 //
-// gala calls GSL once per (n, l, m) term.  Here every special function is
-// produced by its three-term recurrence once per point and reused:
-//   Gegenbauer  n C_n^a = 2 x (n + a - 1) C_{n-1}^a - (n + 2a - 2) C_{n-2}^a
+// gala calls GSL once per (n, l, m) term.  Here the sums are turned round so that
+// a term costs two multiply-adds for the value and four for the gradient, and
+// everything else is formed once per (l, m), per l or per point:
+//
+//   Phi = -G M / r_s sum_l u_l sum_m N_lm P_lm(X) (fS_lm cos m phi + fT_lm sin m phi),
+//   fS_lm = sum_n S_nlm C_n(xi),  u_l = s^l / (1 + s)^(2 l + 1),
+//   N_lm = sqrt((2 l + 1) (l - m)! / (l + m)!)  (4 pi cancels between rho_nl and Y_lm)
+//
+// and the radial derivative needs the same sums over C_{n-1}^{a+1}.  The special
+// functions are three-term recurrences with tabulated coefficients
+// (gx_scf_table.cuh), so no division, root, power or angle is left inside:
+//   Gegenbauer  C_n^a = c1 x C_{n-1}^a - c2 C_{n-2}^a, a = 2 l + 3/2,
+//               C_n^{a+1} = C_{n-2}^{a+1} + (n + a) / a C_n^a
 //   Legendre    (l - m) P_l^m = x (2l - 1) P_{l-1}^m - (l + m - 1) P_{l-2}^m,
 //               P_m^m = (-1)^m (2m - 1)!! (1 - x^2)^{m/2}   (Condon-Shortley, as GSL)
-//   sphPlm      sqrt((2l + 1)/(4 pi) (l - m)!/(l + m)!) P_l^m
-// The terms are summed l-major instead of n-major, so results agree with the
-// term-by-term form to rounding (checked against the oracle in the tests).
+//   cos m phi, sin m phi by the addition theorem from x / R and y / R;
+//   sin theta = R / r (gala's sqrt(1 - X^2) loses digits near the pole).
+// What bounds it is the FP64 pipe: per gradient 4 multiply-adds per (n, l, m), about
+// 3,800 FP64 instructions at nmax = 12, lmax = 8.  131,101 points, potential and
+// gradient, to host arrays: 1.8 ms (34.4 ms when each term formed its own norm,
+// powers and quotients).  As in gala a term whose S and T are both zero is left
+// out, so that a non-finite factor (on the pole, say) does not reach it.
 #pragma once
 
 #include "gx_device.cuh"
+#include "gx_scf_table.cuh"
 
 namespace gx {
 
 constexpr int SCF_MAX_N = 24;   // nmax + 1
 constexpr int SCF_MAX_L = 16;   // lmax + 1
 
-__device__ __forceinline__ double scf_fact(int k) {
-    double f = 1.0;
-    for (int i = 2; i <= k; i++) f *= i;
-    return f;
-}
-
-// P_l^m(X) for all m <= l of one l, given the values of l-1 and l-2 (running
-// recurrence in l).  Arrays are indexed by m.
-__device__ __forceinline__ void scf_legendre_step(int l, double X, double sintheta_pos,
-                                                  const double *Pm1, const double *Pm2, double *P) {
-    // diagonal P_l^l = -(2l-1) sqrt(1-X^2) P_{l-1}^{l-1}
-    for (int m = 0; m <= l; m++) {
-        if (m == l) {
-            P[m] = (l == 0) ? 1.0 : -(2.0 * l - 1.0) * sintheta_pos * Pm1[l - 1];
-        } else if (m == l - 1) {
-            P[m] = X * (2.0 * m + 1.0) * Pm1[m];
-        } else {
-            P[m] = (X * (2.0 * l - 1.0) * Pm1[m] - (l + m - 1.0) * Pm2[m]) / (double)(l - m);
-        }
-    }
-}
-
 // kind 0: value, 1: gradient (accumulated into g), 2: density.
 template <int KIND>
 __device__ __forceinline__ double scf_eval(const double *p, const double *q, double *g) {
-    const double SQRT_FOURPI = 3.544907701811031;
     const double PI = 3.14159265358979323846;
-    const double G = p[0];
+    const double GM = p[0] * p[3];
     const int nmax = (int)p[1];
     const int lmax = (int)p[2];
-    const double M = p[3];
     const double r_s = p[4];
-    const int ncoef = (nmax + 1) * (lmax + 1) * (lmax + 1);
+    const int sn = (lmax + 1) * (lmax + 1);  // coefficients per n
     const double *Snlm = p + 5;
-    const double *Tnlm = p + 5 + ncoef;
+    const double *Tnlm = p + 5 + (nmax + 1) * sn;
 
-    const double r = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]);
-    const double s = r / r_s;
-    const double X = q[2] / r;
-    const double phi = atan2(q[1], q[0]);
-    const double sintheta = sqrt(1 - X * X);
-    const double xi = (s - 1) / (s + 1);
+    const double R2 = fma(q[0], q[0], q[1] * q[1]);
+    const double R = dsqrt(R2), r = dsqrt(fma(q[2], q[2], R2));
+    const double ir = ddiv(1.0, r);
+    const double s = ddiv(r, r_s), s1 = 1.0 + s;
+    const double X = q[2] * ir, st = R * ir;
+    const double i1 = ddiv(1.0, s1);
+    const double xi = (s - 1.0) * i1;
+    const double iR = R2 == 0. ? 0. : ddiv(1.0, R);
+    const double cp = R2 == 0. ? 1. : q[0] * iR, sp = q[1] * iR;  // atan2(0, 0) = 0
 
-    double cosmphi[SCF_MAX_L], sinmphi[SCF_MAX_L];
-    for (int m = 0; m <= lmax; m++) sincos(m * phi, &sinmphi[m], &cosmphi[m]);
+    double C[SCF_MAX_N], D[SCF_MAX_N];                       // C_n^a, C_{n-1}^{a+1}
+    double Pl[SCF_MAX_L], Pl1[SCF_MAX_L], Pl2[SCF_MAX_L];    // P_l^m of this l and the two before
+    double cm[SCF_MAX_L], sm[SCF_MAX_L];
+    cm[0] = 1.;
+    sm[0] = 0.;
+    for (int m = 1; m <= lmax; m++) {
+        cm[m] = fma(cm[m - 1], cp, -(sm[m - 1] * sp));
+        sm[m] = fma(sm[m - 1], cp, cm[m - 1] * sp);
+    }
 
-    double Pl[SCF_MAX_L], Pl1[SCF_MAX_L], Pl2[SCF_MAX_L];
-    for (int m = 0; m < SCF_MAX_L; m++) { Pl[m] = 0.; Pl1[m] = 0.; Pl2[m] = 0.; }
+    const double us = s * i1 * i1;  // u_{l+1} / u_l
+    double u = i1;                  // s^l / (1 + s)^(2 l + 1)
     double acc0 = 0., acc1 = 0., acc2 = 0.;
+    bool angular = false, any = false;
 
     for (int l = 0; l <= lmax; l++) {
-        // Legendre P_l^m (this l) and keep P_{l-1}^m for dY/dtheta
-        for (int m = 0; m < l; m++) { Pl2[m] = Pl1[m]; Pl1[m] = Pl[m]; }
-        scf_legendre_step(l, X, sintheta, Pl1, Pl2, Pl);
-
-        const double a1 = 2 * l + 1.5, a2 = 2 * l + 2.5;
-        const double pow_s_l = pow(s, (double)l);
-        const double pow_s_lm1 = pow(s, (double)(l - 1));
-        double Cn_m2 = 0., Cn_m1 = 0., Cn = 1.;       // C_n^{a1}
-        double Dn_m2 = 0., Dn_m1 = 0., Dn = 1.;       // C_{n-1}^{a2} (Dn is C_{n-1})
-        for (int n = 0; n <= nmax; n++) {
-            // advance Gegenbauer recurrences to index n (C) and n-1 (D)
-            if (n == 0) { Cn = 1.; }
-            else if (n == 1) { Cn_m1 = 1.; Cn = 2. * a1 * xi; }
-            else {
-                Cn_m2 = Cn_m1; Cn_m1 = Cn;
-                Cn = (2. * xi * (n + a1 - 1.) * Cn_m1 - (n + 2. * a1 - 2.) * Cn_m2) / n;
+        // Legendre
+        if (l == 0) {
+            Pl[0] = 1.;
+        } else {
+            for (int m = 0; m < l; m++) {
+                Pl2[m] = Pl1[m];
+                Pl1[m] = Pl[m];
             }
-            const int nd = n - 1;
-            if (nd == 0) { Dn = 1.; }
-            else if (nd == 1) { Dn_m1 = 1.; Dn = 2. * a2 * xi; }
-            else if (nd > 1) {
-                Dn_m2 = Dn_m1; Dn_m1 = Dn;
-                Dn = (2. * xi * (nd + a2 - 1.) * Dn_m1 - (nd + 2. * a2 - 2.) * Dn_m2) / nd;
-            }
+            const double x2 = X * scf::INT[2 * l - 1];
+            for (int m = 0; m < l - 1; m++)
+                Pl[m] = fma(x2, Pl1[m], -(scf::INT[l + m - 1] * Pl2[m])) * scf::INV[l - m];
+            Pl[l - 1] = x2 * Pl1[l - 1];
+            Pl[l] = -scf::INT[2 * l - 1] * st * Pl1[l - 1];
+        }
+        // Gegenbauer (for the density, times K_nl)
+        C[0] = 1.;
+        D[0] = 0.;
+        if (nmax >= 1) {
+            C[1] = scf::GEG1[l][1] * xi;
+            D[1] = 1.;
+        }
+        for (int n = 2; n <= nmax; n++) {
+            C[n] = fma(scf::GEG1[l][n] * xi, C[n - 1], -(scf::GEG2[l][n] * C[n - 2]));
+            if (KIND == 1) D[n] = fma(scf::GEGD[l][n - 1], C[n - 1], D[n - 2]);
+        }
+        if (KIND == 2)
+            for (int n = 0; n <= nmax; n++)
+                C[n] *= 0.5 * n * (n + 4 * l + 3) + (l + 1) * (2 * l + 1);
 
-            double radial, dradial = 0.;
-            if (KIND == 2) {
-                const double Knl = 0.5 * n * (n + 4 * l + 3) + (l + 1) * (2 * l + 1);
-                radial = SQRT_FOURPI * (Knl / (2 * PI) * pow_s_l / (s * pow(1 + s, 2.0 * l + 3)) * Cn);
-            } else {
-                radial = -SQRT_FOURPI * pow_s_l * pow(1 + s, -2.0 * l - 1) * Cn;
+        // sums over n, then over m
+        double fr = 0., fd = 0., ft = 0., fp = 0.;
+        bool anyl = false;
+        for (int m = 0; m <= l; m++) {
+            double sc = 0., tc = 0., sd = 0., td = 0.;
+            long long nz = 0;
+            const double *Sp = Snlm + (m + (lmax + 1) * l), *Tp = Tnlm + (m + (lmax + 1) * l);
+#pragma unroll 4
+            for (int n = 0; n <= nmax; n++) {
+                const double S = __ldg(Sp + n * sn), T = __ldg(Tp + n * sn);
+                const long long b = (__double_as_longlong(S) | __double_as_longlong(T)) << 1;
+                nz |= b;
+                const double c = b ? C[n] : 0., d = b ? D[n] : 0.;
+                sc = fma(S, c, sc);
+                tc = fma(T, c, tc);
                 if (KIND == 1) {
-                    if (n == 0)
-                        dradial = SQRT_FOURPI * pow_s_lm1 * pow(1 + s, -3.0 - 2 * l) * (1 + s) * (l * (-1 + s) + s);
-                    else
-                        dradial = SQRT_FOURPI * pow_s_lm1 * pow(1 + s, -3.0 - 2 * l) *
-                                  (-2 * (3 + 4 * l) * s * Dn + (1 + s) * (l * (-1 + s) + s) * Cn);
+                    sd = fma(S, d, sd);
+                    td = fma(T, d, td);
                 }
             }
-
-            for (int m = 0; m <= l; m++) {
-                const int i = m + (lmax + 1) * (l + (lmax + 1) * n);
-                const double S = Snlm[i], T = Tnlm[i];
-                if ((S == 0.) & (T == 0.)) continue;
-                const double norm = sqrt((double)(2 * l + 1) / (4.0 * PI) * scf_fact(l - m) / scf_fact(l + m));
-                const double Ylm = norm * Pl[m];
-                const double tmp = (S * cosmphi[m] + T * sinmphi[m]);
-                if (KIND != 1) {
-                    acc0 += radial * Ylm * tmp;
-                } else {
-                    double dYlm_dtheta = 0.;
-                    if (l > 0) {
-                        const double Pl1m = (m <= l - 1) ? Pl1[m] : 0.;
-                        const double A = sqrt((double)(2 * l + 1)) / SQRT_FOURPI * sqrt(scf_fact(l - m) / scf_fact(l + m));
-                        dYlm_dtheta = A / sintheta * (l * X * Pl[m] - (l + m) * Pl1m);
-                    }
-                    acc0 += dradial * Ylm * tmp;
-                    acc1 += dYlm_dtheta * radial / s * tmp;
-                    acc2 += ((m == 0) ? 0. : (double)m) * Ylm * radial * (T * cosmphi[m] - S * sinmphi[m]) /
-                            (s * sintheta);
+            if (nz == 0) continue;
+            anyl = true;
+            const double np = scf::YNORM[l][m] * Pl[m];
+            const double fc = fma(sc, cm[m], tc * sm[m]);
+            fr = fma(np, fc, fr);
+            if (KIND == 1) {
+                fd = fma(np, fma(sd, cm[m], td * sm[m]), fd);
+                if (l > 0) {
+                    const double dp = fma(scf::INT[l] * X, Pl[m], m < l ? -(scf::INT[l + m] * Pl1[m]) : 0.);
+                    ft = fma(scf::YNORM[l][m] * dp, fc, ft);
+                }
+                if (m > 0) fp = fma(scf::INT[m] * np, fma(tc, cm[m], -(sc * sm[m])), fp);
+            }
+        }
+        if (anyl) {
+            any = true;
+            if (KIND == 0) acc0 = fma(-u, fr, acc0);
+            if (KIND == 2) acc0 = fma(u, fr, acc0);
+            if (KIND == 1) {
+                // u s^-1 (1 + s)^-2 [(1 + s)(l (s - 1) + s) C - 2 (4 l + 3) s D]
+                const double k = ddiv(u * i1 * i1, s);
+                const double a = s1 * fma(scf::INT[l], s - 1.0, s), b = -2.0 * (4 * l + 3) * s;
+                acc0 = fma(k, fma(a, fr, b * fd), acc0);
+                if (l > 0) {
+                    angular = true;
+                    acc1 = fma(-u, ft, acc1);
+                    acc2 = fma(-u, fp, acc2);
                 }
             }
         }
+        u *= us;
     }
 
-    if (KIND == 0) return acc0 * G * M / r_s;
-    if (KIND == 2) return acc0 * M / (r_s * r_s * r_s);
-    double cosphi, sinphi;
-    sincos(phi, &sinphi, &cosphi);
-    const double gx_ = sintheta * cosphi * acc0 + X * cosphi * acc1 - sinphi * acc2;
-    const double gy_ = sintheta * sinphi * acc0 + X * sinphi * acc1 + cosphi * acc2;
-    const double gz_ = X * acc0 - sintheta * acc1;
-    g[0] += gx_ * G * M / (r_s * r_s);
-    g[1] += gy_ * G * M / (r_s * r_s);
-    g[2] += gz_ * G * M / (r_s * r_s);
+    if (KIND == 0) return ddiv(acc0 * GM, r_s);
+    if (KIND == 2) {
+        // K_nl / (2 pi) s^l / (s (1 + s)^(2 l + 3))
+        return any ? ddiv(acc0 * i1 * i1 * p[3], 2 * PI * s * (r_s * r_s * r_s)) : 0.;
+    }
+    if (!any) return 0.;
+    // the theta and phi parts over s sin theta; without terms of l > 0 gala forms
+    // no quotient for the first and 0 / (s sin theta) for the second
+    const double iss = ddiv(1.0, s * st);
+    acc1 = angular ? acc1 * iss : 0.;
+    acc2 = acc2 * iss;
+    const double f = ddiv(GM, r_s * r_s);
+    g[0] += f * (fma(st * cp, acc0, X * cp * acc1) - sp * acc2);
+    g[1] += f * (fma(st * sp, acc0, X * sp * acc1) + cp * acc2);
+    g[2] += f * fma(X, acc0, -(st * acc1));
     return 0.;
 }
 
