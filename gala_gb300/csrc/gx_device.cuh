@@ -55,8 +55,19 @@ struct DevPot {
     const double *pdev;   // device copy of the packed parameters (may be null)
     const DevComp *cdev;  // component table in device memory (more than
                           // GX_MAX_COMPONENTS components), else null
+    int32_t dbh;          // a disk-bulge-halo composite: see DbhConst
+    int32_t pad;
     DevComp c[GX_MAX_COMPONENTS];
     double p[GX_MAX_INLINE_PARAMS];
+    // Constants of a disk-bulge-halo composite: one or two Hernquist spheres, one
+    // Miyamoto-Nagai disk and one spherical NFW halo, in any order, none shifted or
+    // rotated (a missing second sphere has mass 0).  fast::dbh_gradient evaluates
+    // such a composite in one straight run.
+    struct {
+        double gm1, c1, gm2, c2;  // spheres
+        double gmd, a, b2;        // disk
+        double gmh, irs;          // halo: G m, 1 / r_s
+    } d;
 };
 
 // A large composite seen through its device table: the same members as DevPot

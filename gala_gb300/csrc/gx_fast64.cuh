@@ -9,10 +9,11 @@
 // below instead of gala's literal expressions:
 //
 //   * sqrt, 1/x and ln run on the integer pipe (gx_ipipe.cuh): none of them
-//     costs an FP64-pipe instruction in its usual range.  With the FP32-seeded
-//     Newton forms that stood here before (5, 4 and 14 FP64 instructions) an MW
-//     composite right-hand side took 106 of them; now 47 (DOP853 of 20,011 MW
-//     orbits x 1 Gyr: 232.9 -> 180.3 ms);
+//     costs an FP64-pipe instruction in its usual range.  With FP32-seeded Newton
+//     forms (5, 4 and 14 FP64 instructions) an MW composite right-hand side took
+//     106 of them, with these 47 (DOP853 of 20,011 MW orbits x 1 Gyr: 232.9 ->
+//     180.3 ms), and 33 with one radius and one factor for all its components
+//     (Diag below);
 //   * every a/b becomes a * (1/b) and products and sums are fused (fma);
 //   * gala's formulas are rearranged algebraically where that removes an
 //     operation (the NFW factor v_h^2 / u^3 / r_s^2 is G m / r^3, etc.).
@@ -67,43 +68,72 @@ __device__ __forceinline__ double log_f(double x) {
     return fma(kd, LN2_HI, __ldg(&LOG_TAB[j][1])) + lo_part;
 }
 
-__device__ __forceinline__ double norm3_sq_f(const double *q) { return fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])); }
+// What one evaluation point's components share and add to: the radius (formed when
+// a component first asks for it) and the diagonal factors of the gradient,
+// g = ((F + A0) x, (F + A1) y, (F + A2) z).
+struct Diag {
+    double xy2, r2, r, ir;  // x^2 + y^2, its sum with z^2, the root and its reciprocal
+    double F, A[3];
+    bool have, aniso;
+    __device__ __forceinline__ void init(const double *q) {
+        xy2 = fma(q[0], q[0], q[1] * q[1]);
+        r2 = fma(q[2], q[2], xy2);
+        F = A[0] = A[1] = A[2] = 0.;
+        have = aniso = false;
+    }
+    __device__ __forceinline__ void radius() {
+        if (!have) r = ip::sqrt_rsqrt_n(r2, ir);
+        have = true;
+    }
+    __device__ __forceinline__ void gradient(const double *q, double *g) const {
+        if (aniso) {
+            g[0] = (F + A[0]) * q[0];
+            g[1] = (F + A[1]) * q[1];
+        } else {
+            g[0] = F * q[0];
+            g[1] = F * q[1];
+        }
+        g[2] = (F + A[2]) * q[2];
+    }
+};
 
-// Gradient of one component accumulated into g; the same cases and gala
-// references as comp_gradient in gx_device.cuh.
-template <bool SCF, typename PV>
-__device__ __forceinline__ void comp_gradient_f(const PV &pot, int ci, const double *q, double *g) {
+// Gradient of one closed-form component, added to the diagonal factors; the same
+// cases and gala references as comp_gradient in gx_device.cuh.  Every one of them
+// is a factor times the position, so a spherical component costs 4 to 7 FP64
+// instructions instead of the 13 to 17 it took with a radius, a reciprocal and
+// three accumulations of its own: an MW composite 33 instead of 47.
+template <typename PV>
+__device__ __forceinline__ void comp_gradient_f(const PV &pot, int ci, const double *q, Diag &d) {
     const DevComp &C = pot.c[ci];
     const int type = C.type;
 #define P(k) GX_PARAM(pot, ci, k)
-    double fac;
     switch (type) {
     case GX_POT_NULL:
         return;
-    case GX_POT_KEPLER: {
-        const double r = sqrt_f(norm3_sq_f(q));
-        fac = C.dc[0] * rcp_f(r * r * r);
-        break;
-    }
+    case GX_POT_KEPLER:
+        d.radius();
+        d.F = fma(C.dc[0] * d.ir, d.ir * d.ir, d.F);
+        return;
     case GX_POT_HERNQUIST: {
-        const double r = sqrt_f(norm3_sq_f(q));
-        const double rc = r + P(2);
-        fac = C.dc[0] * rcp_f(rc * rc * r);
-        break;
+        d.radius();
+        const double rc = d.r + P(2);
+        d.F = fma(C.dc[0], rcp_f(rc * rc * d.r), d.F);
+        return;
     }
     case GX_POT_PLUMMER: {
-        const double R2b = norm3_sq_f(q) + C.dc[1];
-        fac = C.dc[0] * rcp_f(R2b * sqrt_f(R2b));
-        break;
+        double i;
+        ip::sqrt_rsqrt_n(d.r2 + C.dc[1], i);
+        d.F = fma(C.dc[0] * i, i * i, d.F);
+        return;
     }
     case GX_POT_MIYAMOTONAGAI: {
-        const double sqrtz = sqrt_f(fma(q[2], q[2], C.dc[1]));
+        double isz, i;
+        const double sqrtz = ip::sqrt_rsqrt_n(fma(q[2], q[2], C.dc[1]), isz);
         const double zd = P(2) + sqrtz;
-        const double W = fma(q[0], q[0], fma(q[1], q[1], zd * zd));
-        fac = C.dc[0] * rcp_f(W * sqrt_f(W));
-        g[0] = fma(fac, q[0], g[0]);
-        g[1] = fma(fac, q[1], g[1]);
-        g[2] = fma(fac * q[2], fma(P(2), rcp_f(sqrtz), 1.), g[2]);
+        ip::sqrt_rsqrt_n(fma(zd, zd, d.xy2), i);
+        const double f = C.dc[0] * i * (i * i);
+        d.F += f;
+        d.A[2] = fma(f, P(2) * isz, d.A[2]);
         return;
     }
     case GX_POT_SPHERICALNFW:
@@ -111,55 +141,103 @@ __device__ __forceinline__ void comp_gradient_f(const PV &pot, int ci, const dou
     case GX_POT_TRIAXIALNFW: {
         // gala: v_h^2 / u^3 / r_s^2 (log(1 + u) - u / (1 + u)) with v_h^2 = G m / r_s
         // and u = m_r / r_s, m_r the (scaled) radius: G m / m_r^3 (...)
-        const bool sph = type == GX_POT_SPHERICALNFW;
-        const double mr2 = sph ? norm3_sq_f(q)
-                               : fma(q[0] * q[0], C.dc[2], fma(q[1] * q[1], C.dc[3], q[2] * q[2] * C.dc[4]));
-        const double mr = sqrt_f(mr2);
-        const double u = mr * C.dc[1];
-        const double mr3 = mr2 * mr, u1 = 1. + u;
-        const double R = rcp_f(mr3 * u1);  // 1 / (m_r^3 (1 + u))
-        fac = C.dc[0] * (u1 * R) * fma(-u, mr3 * R, log_f(u1));
-        if (sph) break;
-        g[0] = fma(fac * C.dc[2], q[0], g[0]);
-        g[1] = fma(fac * C.dc[3], q[1], g[1]);
-        g[2] = fma(fac * C.dc[4], q[2], g[2]);
-        return;
-    }
-    case GX_POT_SCF:
-        if constexpr (SCF) {
-            scf_gradient_dev(pot.pdev + pot.c[ci].poff, q, g);
+        double mr, im;
+        if (type == GX_POT_SPHERICALNFW) {
+            d.radius();
+            mr = d.r;
+            im = d.ir;
+        } else {
+            mr = ip::sqrt_rsqrt_n(fma(q[0] * q[0], C.dc[2], fma(q[1] * q[1], C.dc[3], q[2] * q[2] * C.dc[4])), im);
+        }
+        const double u = mr * C.dc[1], u1 = 1. + u;
+        const double f = C.dc[0] * im * (im * im) * fma(-u, rcp_f(u1), log_f(u1));
+        if (type == GX_POT_SPHERICALNFW) {
+            d.F += f;
             return;
         }
-        fac = __longlong_as_double(0x7ff8000000000000LL);
-        break;
-    default: {
-        const double nan = __longlong_as_double(0x7ff8000000000000LL);
-        g[0] = nan; g[1] = nan; g[2] = nan;
+        d.aniso = true;
+        d.A[0] = fma(f, C.dc[2], d.A[0]);
+        d.A[1] = fma(f, C.dc[3], d.A[1]);
+        d.A[2] = fma(f, C.dc[4], d.A[2]);
         return;
     }
+    default:
+        d.F = __longlong_as_double(0x7ff8000000000000LL);
+        return;
     }
-    g[0] = fma(fac, q[0], g[0]);
-    g[1] = fma(fac, q[1], g[1]);
-    g[2] = fma(fac, q[2], g[2]);
 #undef P
 }
 
 template <bool SCF, typename PV>
 __device__ __forceinline__ void potential_gradient_ft(const PV &pot, const double *q, double *g) {
-    g[0] = 0.; g[1] = 0.; g[2] = 0.;
+    Diag d;
+    d.init(q);
+    double gs[3] = {0., 0., 0.};  // shifted or rotated components and SCF
+    bool extra = false;
     for (int i = 0; i < pot.ncomp; i++) {
-        if (pot.c[i].do_sr == 0) {
-            comp_gradient_f<SCF>(pot, i, q, g);
+        const DevComp &c = pot.c[i];
+        if constexpr (SCF) {
+            if (c.type == GX_POT_SCF && c.do_sr == 0) {
+                scf_gradient_dev(pot.pdev + c.poff, q, gs);
+                extra = true;
+                continue;
+            }
+        }
+        if (c.do_sr == 0) {
+            comp_gradient_f(pot, i, q, d);
         } else {
-            const DevComp &c = pot.c[i];
             double qt[3], gt[3] = {0., 0., 0.};
             shift_rotate(c, q, qt);
-            comp_gradient_f<SCF>(pot, i, qt, gt);
-            g[0] += fma(c.R[0], gt[0], fma(c.R[3], gt[1], c.R[6] * gt[2]));
-            g[1] += fma(c.R[1], gt[0], fma(c.R[4], gt[1], c.R[7] * gt[2]));
-            g[2] += fma(c.R[2], gt[0], fma(c.R[5], gt[1], c.R[8] * gt[2]));
+            if constexpr (SCF) {
+                if (c.type == GX_POT_SCF) scf_gradient_dev(pot.pdev + c.poff, qt, gt);
+            }
+            if (c.type != GX_POT_SCF) {
+                Diag dt;
+                dt.init(qt);
+                comp_gradient_f(pot, i, qt, dt);
+                dt.gradient(qt, gt);
+            }
+            gs[0] += fma(c.R[0], gt[0], fma(c.R[3], gt[1], c.R[6] * gt[2]));
+            gs[1] += fma(c.R[1], gt[0], fma(c.R[4], gt[1], c.R[7] * gt[2]));
+            gs[2] += fma(c.R[2], gt[0], fma(c.R[5], gt[1], c.R[8] * gt[2]));
+            extra = true;
         }
     }
+    d.gradient(q, g);
+    if (extra)
+        for (int k = 0; k < 3; k++) g[k] += gs[k];
+}
+
+// Gradient of a disk-bulge-halo composite (DevPot::d) in one straight run: 29 FP64
+// instructions, and the two square roots, the inverse root, the three reciprocals
+// and the logarithm on the integer pipe side by side instead of one after the
+// other behind the component loop's branches (with it the DOP853 population of 20,011
+// orbits x 1 Gyr takes 84 ms, without 134).  False where an argument is outside the integer forms' range (a point
+// within 2^-6 r_s of the centre, a non-finite position): the general form then
+// serves.
+__device__ __forceinline__ bool dbh_gradient(const DevPot &pot, const double *q, double *g) {
+    const double xy2 = fma(q[0], q[0], q[1] * q[1]);
+    const double r2 = fma(q[2], q[2], xy2);
+    const double w = fma(q[2], q[2], pot.d.b2);
+    double ir, isz;
+    const double r = ip::sqrt_rsqrt_u(r2, ir), sz = ip::sqrt_rsqrt_u(w, isz);
+    const double d1 = r + pot.d.c1, d2 = r + pot.d.c2;
+    const double u = r * pot.d.irs, u1 = 1. + u;
+    const double zd = pot.d.a + sz;
+    const double W = fma(zd, zd, xy2);
+    const bool ok = ip::ok_sqrt(r2) & ip::ok_sqrt(w) & ip::ok_rcp(d1) & ip::ok_rcp(d2) & ip::ok_sqrt(W) & ip::ln_range(u1) &
+                    ip::ok_rcp(u1);
+    const double iW = ip::rsqrt_u(W);
+    const double t1 = ip::rcp_u(d1), t2 = ip::rcp_u(d2), iu = ip::rcp_u(u1);
+    const double L = ip::ln_n(u1);
+    // spheres and halo share a factor 1 / r: G m / (r + c)^2 and G m (L - u / (1 + u)) / r^2
+    const double s = fma(pot.d.gmh * (ir * ir), fma(-u, iu, L), fma(pot.d.gm1, t1 * t1, pot.d.gm2 * (t2 * t2)));
+    const double f = pot.d.gmd * iW * (iW * iW);
+    const double F = fma(ir, s, f);
+    g[0] = F * q[0];
+    g[1] = F * q[1];
+    g[2] = fma(f, pot.d.a * isz, F) * q[2];
+    return ok;
 }
 
 // A large composite (device component table) takes gala's own expressions: the
@@ -171,7 +249,20 @@ __device__ __forceinline__ void potential_gradient_f(const DevPot &pot, const do
         potential_gradient_t<SCF, false>(table_view(pot), q, g);
         return;
     }
+    if constexpr (!SCF) {
+        if (pot.dbh && dbh_gradient(pot, q, g)) return;
+    }
     potential_gradient_ft<SCF>(pot, q, g);
+}
+
+// Acceleration in a static frame.
+template <bool SCF>
+__device__ __noinline__ V3 accel_call_f(const DevPot &pot, V3 q) {
+    double g[3];
+    potential_gradient_f<SCF>(pot, q.v, g);
+    V3 a;
+    for (int c = 0; c < 3; c++) a.v[c] = -g[c];
+    return a;
 }
 
 // Hamilton's equations (hamiltonian_rhs in gx_device.cuh) with the fast force.

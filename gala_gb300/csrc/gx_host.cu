@@ -84,6 +84,34 @@ static bool regular_component(int type, const double *P, int do_sr) {
     }
 }
 
+// Whether the packed components are a disk-bulge-halo composite; its constants.
+static void pack_dbh(DevPot *out) {
+    out->d.gm2 = 0.;
+    out->d.c2 = 1.;
+    int nh = 0, nd = 0, nn = 0;
+    for (int i = 0; i < out->ncomp; i++) {
+        const DevComp &c = out->c[i];
+        if (c.do_sr) return;
+        if (c.type == GX_POT_HERNQUIST) {
+            (nh == 0 ? out->d.gm1 : out->d.gm2) = c.dc[0];
+            (nh == 0 ? out->d.c1 : out->d.c2) = out->p[c.poff + 2];
+            nh++;
+        } else if (c.type == GX_POT_MIYAMOTONAGAI) {
+            out->d.gmd = c.dc[0];
+            out->d.a = out->p[c.poff + 2];
+            out->d.b2 = c.dc[1];
+            nd++;
+        } else if (c.type == GX_POT_SPHERICALNFW) {
+            out->d.gmh = c.dc[0];
+            out->d.irs = c.dc[1];
+            nn++;
+        } else {
+            return;
+        }
+    }
+    out->dbh = (nh == 1 || nh == 2) && nd == 1 && nn == 1;
+}
+
 // Validate the descriptor's header and component i; *need = the doubles its type uses.
 static int check_header(const gx_potential *pot) {
     GX_CHECK_ARG(pot != nullptr, "potential descriptor is NULL");
@@ -163,6 +191,7 @@ int pack_potential(const gx_potential *pot, DevPot *out) {
         if (!regular_component(c.type, pot->params + c.param_offset, d.do_sr)) out->regular = 0;
     }
     out->n_inline = ninl;
+    pack_dbh(out);
     return GX_OK;
 }
 

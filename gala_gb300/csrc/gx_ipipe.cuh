@@ -224,29 +224,40 @@ __device__ __forceinline__ double sqrt_n(double x) {
     const SqrtArg a = sqrt_arg(hi, lo);
     return pack53(sqrt53(a.v, rsqrt63(a.v, rsqrt_seed(a.fb))), a.hbits);
 }
+// The forms named _u take any bits and are right where ok_ says so; a straight
+// run of them leaves the compiler free to interleave their dependent chains (190
+// to 430 cycles each alone), which a branch in each would forbid.
+
 // sqrt(x) (returned) and 1 / sqrt(x), each within 0.51 ulp, from one core.
-__device__ __forceinline__ double sqrt_rsqrt_n(double x, double &rs) {
-    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    if (!normal_pos(hi)) {
-        const double s = sqrt(x);
-        rs = 1.0 / s;
-        return s;
-    }
-    const SqrtArg a = sqrt_arg(hi, lo);
+__device__ __forceinline__ bool ok_sqrt(double x) { return normal_pos((uint32_t)__double2hiint(x)); }
+__device__ __forceinline__ double sqrt_rsqrt_u(double x, double &rs) {
+    const SqrtArg a = sqrt_arg((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x));
     const uint64_t y = rsqrt63(a.v, rsqrt_seed(a.fb));
     // 1 / sqrt(x) = y 2^-h, y in (0.5, 1] at 2^-63: R = y 2^53 in [2^52, 2^53], exponent -h - 1
     rs = pack53((y + 512) >> 10, (2u * 1022u - 1u) * (1u << 20) - a.hbits);
     return pack53(sqrt53(a.v, y), a.hbits);
 }
+__device__ __forceinline__ double rsqrt_u(double x) {
+    double rs;
+    sqrt_rsqrt_u(x, rs);
+    return rs;
+}
+__device__ __forceinline__ double sqrt_rsqrt_n(double x, double &rs) {
+    if (ok_sqrt(x)) return sqrt_rsqrt_u(x, rs);
+    const double s = sqrt(x);
+    rs = 1.0 / s;
+    return s;
+}
 // 1/x within 0.51 ulp.
-__device__ __forceinline__ double rcp_n(double x) {
+__device__ __forceinline__ bool ok_rcp(double x) { return mid_range((uint32_t)__double2hiint(x)); }
+__device__ __forceinline__ double rcp_u(double x) {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    if (!mid_range(hi)) return 1.0 / x;
     const Mant m = mant63(hi, lo);
     const uint64_t y = rcp63(m.hi, m.lo, rcp_seed(0x3f800000u | top23(hi, lo)));
     const uint32_t eb = (2044u << 20) - (hi & 0x7ff00000u);  // -k - 1 + 1022
     return pack53((y + 512) >> 10, eb | (hi & 0x80000000u));
 }
+__device__ __forceinline__ double rcp_n(double x) { return ok_rcp(x) ? rcp_u(x) : 1.0 / x; }
 // IEEE a / b.
 __device__ __forceinline__ double div_rn(double a, double b) {
     const uint32_t ah = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
