@@ -55,7 +55,9 @@ struct DevPot {
     const double *pdev;   // device copy of the packed parameters (may be null)
     const DevComp *cdev;  // component table in device memory (more than
                           // GX_MAX_COMPONENTS components), else null
-    int32_t dbh;          // a disk-bulge-halo composite: see DbhConst
+    int32_t dbh;          // a disk-bulge-halo composite: see d
+    int32_t dbh_order;    // and its order: 1 spheres, disk, halo; 2 disk, spheres, halo; 0 another
+    int32_t sphere;       // one unshifted Hernquist or Plummer sphere: its type (d.gm1; d.c1 = c or b^2), else 0
     int32_t pad;
     DevComp c[GX_MAX_COMPONENTS];
     double p[GX_MAX_INLINE_PARAMS];
@@ -67,6 +69,7 @@ struct DevPot {
         double gm1, c1, gm2, c2;  // spheres
         double gmd, a, b2;        // disk
         double gmh, irs;          // halo: G m, 1 / r_s
+        double vh2, rs, rs2;      // halo, as gala's expressions take it: G m / r_s, r_s, r_s^2
     } d;
 };
 
@@ -282,6 +285,71 @@ __device__ __forceinline__ void comp_gradient(const PV &pot, int ci, const doubl
 #undef P
 }
 
+// comp_gradient for one axis: the component `axis` of the gradient is increased in
+// g, with q the coordinate and s0, s1, s2 the squares of all three (the same
+// expressions as above, so the same bits).
+template <typename PV>
+__device__ __forceinline__ void comp_gradient_axis(const PV &pot, int ci, double s0, double s1, double s2, double q, int axis,
+                                                   double &g, Radius &R) {
+    const DevComp &C = pot.c[ci];
+#define P(k) GX_PARAM(pot, ci, k)
+    double fac;
+    R.s = s0 + s1 + s2;
+    if (R.have == 0) R.have = 1;
+    const double *none = nullptr;
+    switch (C.type) {
+    case GX_POT_NULL:
+        return;
+    case GX_POT_KEPLER:
+        fac = ddiv(C.dc[0], cube(R.root(none)));
+        break;
+    case GX_POT_HERNQUIST: {
+        const double r = R.root(none);
+        fac = ddiv(C.dc[0], (r + P(2)) * (r + P(2)) * r);
+        break;
+    }
+    case GX_POT_PLUMMER: {
+        const double R2b = R.s + C.dc[1];
+        fac = ddiv(ddiv(C.dc[0], dsqrt(R2b)), R2b);
+        break;
+    }
+    case GX_POT_MIYAMOTONAGAI: {
+        const double sqrtz = dsqrt(s2 + C.dc[1]);
+        const double zd = P(2) + sqrtz;
+        fac = C.dc[0] * pow_m1p5(s0 + s1 + zd * zd);
+        if (axis == 2)
+            g = g + fac * q * (1. + ddiv(P(2), sqrtz));
+        else
+            g = g + fac * q;
+        return;
+    }
+    case GX_POT_SPHERICALNFW:
+    case GX_POT_FLATTENEDNFW:
+    case GX_POT_TRIAXIALNFW: {
+        double m;
+        if (C.type == GX_POT_SPHERICALNFW)
+            m = R.root(none);
+        else if (C.type == GX_POT_FLATTENEDNFW)
+            m = dsqrt(s0 + s1 + ddiv(s2, P(5) * P(5)));
+        else
+            m = dsqrt(ddiv(s0, P(3) * P(3)) + ddiv(s1, P(4) * P(4)) + ddiv(s2, P(5) * P(5)));
+        const double u = ddiv(m, P(2)), u1 = 1 + u;
+        fac = ddiv(ddiv(C.dc[5], u * u * u), C.dc[6]) * (dlog<false>(u1) - ddiv(u, u1));
+        if (C.type == GX_POT_TRIAXIALNFW || (C.type == GX_POT_FLATTENEDNFW && axis == 2)) {
+            const double a = P(3 + axis);
+            g = g + ddiv(fac * q, a * a);
+            return;
+        }
+        break;
+    }
+    default:
+        g = __longlong_as_double(0x7ff8000000000000LL);
+        return;
+    }
+    g = g + fac * q;
+#undef P
+}
+
 // Density of one component (kepler_density :78-88, hernquist_density :235-244,
 // plummer_density :316-324, miyamotonagai_density :1314-1332,
 // sphericalnfw_density :852-864).  Flattened/triaxial NFW have no density in
@@ -398,6 +466,47 @@ __device__ __forceinline__ void potential_gradient_t(const PV &pot, const double
     }
 }
 
+// The factors of a disk-bulge-halo composite's gradient in gala's expressions, in
+// one straight run (see fast::dbh_gradient): spheres f1, f2, disk fd with mz on
+// its z component, halo fn; s0, s1, s2 are the squares of the coordinates.  False
+// where an argument is outside the integer forms' range.  The bits are those of
+// comp_gradient; side by side the chains take 16,384 uneven FP64 orbits from 35.5
+// to 22.0 ms.
+template <bool LIBLN>
+__device__ __forceinline__ bool dbh_factors(const DevPot &pot, double s0, double s1, double s2, double &f1, double &f2,
+                                            double &fd, double &mz, double &fn) {
+    const double xy2 = s0 + s1;
+    const double r2 = xy2 + s2, w = s2 + pot.d.b2;
+    const double r = ip::sqrt_rn_u(r2), sz = ip::sqrt_rn_u(w);
+    const double d1 = (r + pot.d.c1) * (r + pot.d.c1) * r, d2 = (r + pot.d.c2) * (r + pot.d.c2) * r;
+    const double u = ip::div_rn_u(r, pot.d.rs);
+    const double zd = pot.d.a + sz;
+    const double W = xy2 + zd * zd;
+    const double sW = ip::sqrt_rn_u(W), W3 = W * sW;
+    const double u1 = 1 + u, u3 = u * u * u;
+    const bool ok = ip::ok_sqrt(r2) & ip::ok_sqrt(w) & ip::ok_sqrt(W) & ip::ok_div(pot.d.gm1, d1) & ip::ok_rcp(d2) &
+                    ip::ok_div(r, pot.d.rs) & ip::ok_rcp(W3) & ip::ok_div(pot.d.a, sz) & ip::ln_range(u1) & ip::ok_rcp(u1) &
+                    ip::ok_div(pot.d.vh2, u3) & ip::ok_rcp(pot.d.rs2);
+    f1 = ip::div_rn_u(pot.d.gm1, d1);
+    f2 = __double_as_longlong(pot.d.gm2) == 0 ? 0. : ip::div_rn_u(pot.d.gm2, d2);
+    fd = pot.d.gmd * ip::div_rn_u(1.0, W3);
+    mz = 1. + ip::div_rn_u(pot.d.a, sz);
+    const double L = LIBLN ? log(u1) : ip::ln_n(u1);
+    const double v = ip::div_rn_u(pot.d.vh2, u3);
+    fn = ip::div_rn_u(v, pot.d.rs2) * (L - ip::div_rn_u(u, u1));
+    return ok & ip::ok_rcp(v);
+}
+
+// One component of the gradient of such a composite from its factors, summed in
+// the composite's order.
+__device__ __forceinline__ double dbh_sum(int order, double q, double f1, double f2, double fd, double mz, double fn) {
+    const double gd = fd * q * mz;
+    const double a = order == 1 ? 0. + f1 * q : 0. + gd;
+    const double b = order == 1 ? a + f2 * q : a + f1 * q;
+    const double c = order == 1 ? b + gd : b + f2 * q;
+    return c + fn * q;
+}
+
 // The descriptor's components: the by-value array, or the device table of a
 // large composite (the branch is uniform over the grid).
 template <bool SCF>
@@ -415,6 +524,17 @@ __device__ __forceinline__ void potential_gradient(const DevPot &pot, const doub
     if (pot.cdev) {
         potential_gradient_t<SCF, LIBLN>(table_view(pot), q, g);
         return;
+    }
+    if constexpr (!SCF) {
+        if (pot.dbh_order) {
+            double f1, f2, fd, mz, fn;
+            if (dbh_factors<LIBLN>(pot, q[0] * q[0], q[1] * q[1], q[2] * q[2], f1, f2, fd, mz, fn)) {
+                g[0] = dbh_sum(pot.dbh_order, q[0], f1, f2, fd, 1., fn);
+                g[1] = dbh_sum(pot.dbh_order, q[1], f1, f2, fd, 1., fn);
+                g[2] = dbh_sum(pot.dbh_order, q[2], f1, f2, fd, mz, fn);
+                return;
+            }
+        }
     }
     potential_gradient_t<SCF, LIBLN>(pot, q, g);
 }
@@ -482,6 +602,107 @@ __device__ __noinline__ V3 gradient_call(const DevPot &pot, V3 q) {
     V3 g;
     potential_gradient<SCF, LIBLN>(pot, q.v, g.v);
     return g;
+}
+
+// Lane k's value in each group of four lanes.
+__device__ __forceinline__ double quad(double v, int k) { return __shfl_sync(0xffffffffu, v, k, 4); }
+
+// The gradient's component `axis` at a point held by four lanes of a warp (lane c of
+// the group holds coordinate min(c, 2); axis is the lane's).  Closed-form components
+// in the by-value descriptor only.  All 32 lanes of the warp take part: with a mask
+// per group every shuffle would wait on a synchronisation of its own.
+static __device__ __noinline__ double gradient_axis_call(const DevPot &pot, double q, int axis) {
+    const double s = q * q;
+    const double s0 = quad(s, 0), s1 = quad(s, 1), s2 = quad(s, 2);
+    double g = 0.;
+    Radius R;
+    R.have = 0;
+    for (int i = 0; i < pot.ncomp; i++) {
+        if (pot.c[i].do_sr == 0) {
+            comp_gradient_axis(pot, i, s0, s1, s2, q, axis, g, R);
+        } else {
+            const DevComp &c = pot.c[i];
+            double qf[3], qt[3], gt[3] = {0., 0., 0.};
+            for (int k = 0; k < 3; k++) qf[k] = quad(q, k);
+            Radius Rt;
+            Rt.have = 0;
+            shift_rotate(c, qf, qt);
+            comp_gradient<false, false>(pot, i, qt, gt, Rt);
+            g += c.R[axis] * gt[0] + c.R[3 + axis] * gt[1] + c.R[6 + axis] * gt[2];
+        }
+    }
+    return g;
+}
+
+// Straight runs of the same for the composites that have one: MODE 1 a Hernquist
+// sphere, 2 and 3 a disk-bulge-halo composite (dbh_order 1 and 2); 0 the general
+// form.  Constants that differ by lane are read once per launch (AxisLane), and
+// choices between lanes are selections: a branch would end the run in which the
+// integer chains overlap.
+struct AxisLane {
+    double cc, num;  // the lane's sphere radius and numerator
+    bool first, sphere, halo, z;
+};
+__device__ __forceinline__ double pick(bool p, double a, double b) {
+    return __hiloint2double(p ? __double2hiint(a) : __double2hiint(b), p ? __double2loint(a) : __double2loint(b));
+}
+__device__ __forceinline__ AxisLane axis_lane(const DevPot &pot) {
+    const int c = threadIdx.x & 3;
+    AxisLane L;
+    L.cc = c == 0 ? pot.d.c1 : pot.d.c2;
+    // a missing second sphere: 1 / d, taken as 0 below
+    L.num = c == 0 ? pot.d.gm1 : c == 1 ? (pot.d.gm2 == 0. ? 1. : pot.d.gm2) : pot.d.a;
+    L.first = c == 0;
+    L.sphere = c < 2;
+    L.halo = c == 2;
+    L.z = c >= 2;
+    return L;
+}
+
+// False, for the whole warp, where an argument of a lane that counts is outside the
+// integer forms' range: the caller goes on with the general form (a call here would
+// make every value alive around it spill).
+template <int MODE>
+__device__ __forceinline__ bool gradient_axis(const DevPot &pot, const AxisLane &A, bool counts, double q, double &g) {
+    const double s = q * q;
+    const double s0 = quad(s, 0), s1 = quad(s, 1), s2 = quad(s, 2);
+    bool ok;
+    if constexpr (MODE == 1) {
+        const double r2 = s0 + s1 + s2;
+        const double r = ip::sqrt_rn_u(r2);
+        const double d = (r + pot.d.c1) * (r + pot.d.c1) * r;
+        ok = ip::ok_sqrt(r2) & ip::ok_div(pot.d.gm1, d);
+        g = 0. + ip::div_rn_u(pot.d.gm1, d) * q;
+    } else {
+        // dbh_factors with the integer work shared out: of two square roots, and of
+        // four and three quotients, each lane forms one
+        const double xy2 = s0 + s1;
+        const double a1 = pick(A.first || A.halo, xy2 + s2, s2 + pot.d.b2);
+        const double q1 = ip::sqrt_rn_u(a1);
+        const double r = quad(q1, 0), sz = quad(q1, 1);
+        const double rc = r + A.cc;
+        const double num = pick(A.halo, r, A.num), den = pick(A.sphere, rc * rc * r, pick(A.halo, pot.d.rs, sz));
+        const double zd = pot.d.a + sz;
+        const double W = xy2 + zd * zd;
+        const double q2 = ip::div_rn_u(num, den);
+        const double W3 = W * ip::sqrt_rn_u(W);
+        const double f1 = quad(q2, 0), f2s = quad(q2, 1);
+        const double u = quad(q2, 2), mz = 1. + quad(q2, 3);
+        const double f2 = pick(__double_as_longlong(pot.d.gm2) == 0, 0., f2s);
+        const double u1 = 1 + u, u3 = u * u * u;
+        const double num3 = pick(A.z, u, pick(A.first, 1.0, pot.d.vh2));
+        const double den3 = pick(A.z, u1, pick(A.first, W3, u3));
+        const double q3 = ip::div_rn_u(num3, den3);
+        const double L = ip::ln_n(u1);
+        const double v = quad(q3, 1);
+        const double fd = pot.d.gmd * quad(q3, 0);
+        const double fn = ip::div_rn_u(v, pot.d.rs2) * (L - quad(q3, 2));
+        ok = ip::ok_sqrt(a1) & ip::ok_div(num, den) & ip::ok_sqrt(W) & ip::ok_div(num3, den3) & ip::ln_range(u1) &
+             ip::ok_div(v, pot.d.rs2);
+        const double gd = fd * q * pick(A.z, mz, 1.0);
+        g = MODE == 2 ? 0. + f1 * q + f2 * q + gd + fn * q : 0. + gd + f1 * q + f2 * q + fn * q;
+    }
+    return __all_sync(0xffffffffu, ok | !counts);
 }
 
 template <bool SCF>

@@ -8,12 +8,13 @@
 //   leapfrog  c_init_velocity / c_leapfrog_step (leapfrog.pyx:24-51,99-116)
 //   ruth4     c_ruth4_step with gala's coefficients (ruth4.pyx:24-35,65-78,98-108)
 // What bounds them is the FP64 pipe: one warp alone on a scheduler retires an
-// FP64 instruction per 64 cycles whatever it depends on.  Roots and quotients on
-// the integer pipe (gx_device.cuh), Ruth4's zero-weight gradient left out where
-// it is certainly finite, and Leapfrog's synchronised velocity formed only where
-// it is stored took 16,384 uneven orbits (100 to 2,000 steps) from 69.8 to 35.5 ms
-// and 1,024 Hernquist orbits x 1,000 stored steps from 2.37 to 1.80 ms, with the
-// same bits (ln, in NFW, within an ulp).
+// FP64 instruction per 64 cycles whatever it depends on, and the SM's unit one per
+// 19.  Roots and quotients run on the integer pipe (gx_device.cuh), Ruth4's
+// zero-weight gradient is left out where it is certainly finite, Leapfrog's
+// synchronised velocity is formed only where it is stored, and few orbits take four
+// lanes each: 16,384 uneven orbits (100 to 2,000 steps) 69.8 -> 11.9 ms, 1,024
+// Hernquist orbits x 1,000 stored steps 2.37 -> 0.73 ms, with the same bits (ln, in
+// NFW, within an ulp).
 #include "gx_host.h"
 #include "gx_queue.cuh"
 #include "gx_scf.cuh"
@@ -122,6 +123,156 @@ __global__ void __launch_bounds__(128, 1) ruth4_kernel(const __grid_constant__ D
 }
 
 // ---------------------------------------------------------------------------
+// The same two integrators for few orbits: four lanes per orbit, one coordinate
+// each (the fourth repeats z).  An FP64 instruction costs a warp 64 cycles whether
+// one lane or 32 take part, and few orbits leave most of the schedulers without a
+// warp, so the three coordinates of an orbit go side by side: per Leapfrog step of a
+// Hernquist orbit 15 FP64 instructions instead of 36, of the MW composite 36 instead
+// of 66.  The operations and their order are those above, so the bits are too.
+// The line lies at one warp per scheduler (8 orbits per warp, 4 schedulers per SM):
+// a Ruth4 step of 4,864 MW orbits takes 5.0 us, of 6,000 with one lane per orbit 10.9;
+// 1,024 Hernquist orbits x 1,000 stored Leapfrog steps 1.80 -> 0.73 ms.
+// ---------------------------------------------------------------------------
+// gradient_axis's MODE for a potential.
+static int axis_mode(const DevPot &dp) { return dp.sphere == GX_POT_HERNQUIST ? 1 : dp.dbh_order ? 1 + dp.dbh_order : 0; }
+
+// Steps of the orbits of a warp's eight groups of four lanes, (x, v) the lane's
+// coordinate: n_steps for each (EVEN, the same for all) or the lane's own ns <= n_steps,
+// after which it goes along without moving.  store(j) after step j when SAVE.  The
+// straight run serves from the first step on; where it declines a point, the warp is
+// finished with the general form.
+template <int MODE, bool RUTH, bool EVEN, bool SAVE, typename Store>
+__device__ __forceinline__ void axis_run(const DevPot &pot, const AxisLane &A, const Ruth4Coef &co, double dt, int64_t n_steps,
+                                         int64_t ns, int axis, double &x, double &v, Store store) {
+    double g;
+    if (!RUTH) {
+        // the gradient at x belongs to the start (at = 0) or to step `at`, whose drift is done
+        int64_t at = 0;
+        double vh = v;
+        if constexpr (MODE != 0) {
+            if (gradient_axis<MODE>(pot, A, EVEN || ns > 0, x, g)) {
+                vh = half_kick(v, g * dt);
+                for (;;) {
+                    if (++at > n_steps) return;
+                    const bool on = EVEN || at <= ns;
+                    x = pick(on, x + vh * dt, x);
+                    if (!gradient_axis<MODE>(pot, A, on, x, g)) break;
+                    const double gd = g * dt;
+                    if (SAVE || at == (EVEN ? n_steps : ns)) v = half_kick(vh, gd);
+                    vh = pick(on, vh - gd, vh);
+                    if (SAVE) store(at);
+                }
+            }
+        }
+        for (;;) {
+            const double gd = gradient_axis_call(pot, x, axis) * dt;
+            if (at == 0) {
+                vh = half_kick(v, gd);
+            } else {
+                if (SAVE || at == (EVEN ? n_steps : ns)) v = half_kick(vh, gd);
+                vh = pick(EVEN || at <= ns, vh - gd, vh);
+                if (SAVE) store(at);
+            }
+            if (++at > n_steps) return;
+            x = pick(EVEN || at <= ns, x + vh * dt, x);
+        }
+    } else {
+        const bool regular = ordinary(dt) && pot.regular;
+        // sub-step 0's zero-weight gradient, as in ruth4_step (the largest coordinate of the orbit)
+        auto zero = [&](bool on) {
+            unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            return __all_sync(0xffffffffu, (regular && m - (923u << 20) < (200u << 20)) || !on);
+        };
+        int64_t j = 1;
+        int s = 0;  // the sub-step to do
+        if constexpr (MODE != 0) {
+            bool ok = true;
+            while (j <= n_steps && ok) {
+                const bool on = EVEN || j <= ns;
+                if (!zero(on)) break;
+                x = pick(on, x + co.c[0] * v * dt, x);
+#pragma unroll 1
+                for (s = 1; s < 4; s++) {
+                    ok = gradient_axis<MODE>(pot, A, on, x, g);
+                    if (!ok) break;
+                    v = pick(on, v - co.d[s] * g * dt, v);
+                    x = pick(on, x + co.c[s] * v * dt, x);
+                }
+                if (!ok) break;
+                s = 0;
+                if (SAVE) store(j);
+                j++;
+            }
+        }
+        for (; j <= n_steps; j++) {
+            const bool on = EVEN || j <= ns;
+#pragma unroll 1
+            for (; s < 4; s++) {
+                if (s > 0 || !zero(on)) {
+                    g = gradient_axis_call(pot, x, axis);
+                    v = pick(on, v - co.d[s] * g * dt, v);
+                }
+                x = pick(on, x + co.c[s] * v * dt, x);
+            }
+            s = 0;
+            if (SAVE) store(j);
+        }
+    }
+}
+
+template <int MODE, bool RUTH, bool SAVE_ALL>
+__global__ void __launch_bounds__(32) fixed_axis_kernel(const __grid_constant__ DevPot pot, Ruth4Coef co,
+                                                        const double *__restrict__ w0, int64_t n,
+                                                        const double *__restrict__ t, int64_t ntimes,
+                                                        double *__restrict__ out) {
+    const int lane = threadIdx.x, c = lane & 3, axis = c < 2 ? c : 2;
+    const int64_t orbit = (int64_t)blockIdx.x * 8 + (lane >> 2);
+    const bool keep = orbit < n && c < 3;
+    const int64_t i = orbit < n ? orbit : n - 1;
+    double x = w0[axis * n + i], v = w0[(3 + axis) * n + i];
+    double *ox = out + (SAVE_ALL ? axis * ntimes : axis) * n + i;
+    double *ov = out + (SAVE_ALL ? (3 + axis) * ntimes : 3 + axis) * n + i;
+    auto store = [&](int64_t j) {
+        if (keep) {
+            __stcs(ox + j * n, x);
+            __stcs(ov + j * n, v);
+        }
+    };
+    if (SAVE_ALL) store(0);
+    axis_run<MODE, RUTH, true, SAVE_ALL>(pot, axis_lane(pot), co, t[1] - t[0], ntimes - 1, ntimes - 1, axis, x, v, store);
+    if (!SAVE_ALL) store(0);
+}
+
+template <bool RUTH>
+static int launch_axis(const DevPot &dp, const Ruth4Coef &co, const double *w0, int64_t n, const double *t, int64_t ntimes,
+                       bool save_all, double *out, cudaStream_t st, const char *name) {
+    const unsigned g8 = (unsigned)((n + 7) / 8);
+    switch ((axis_mode(dp) << 1) | (save_all ? 1 : 0)) {
+#define GX_CASE(m)                                                                                       \
+    case 2 * m: fixed_axis_kernel<m, RUTH, false><<<g8, 32, 0, st>>>(dp, co, w0, n, t, ntimes, out); break; \
+    case 2 * m + 1: fixed_axis_kernel<m, RUTH, true><<<g8, 32, 0, st>>>(dp, co, w0, n, t, ntimes, out); break
+        GX_CASE(0);
+        GX_CASE(1);
+        GX_CASE(2);
+        GX_CASE(3);
+#undef GX_CASE
+    }
+    return check_launch(name);
+}
+
+static int multiprocessors() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return sms;
+}
+
+// Whether few enough orbits for one coordinate per lane.
+static bool few_orbits(const DevPot &dp, int64_t n) { return !dp.has_scf && !dp.cdev && n <= (int64_t)32 * multiprocessors(); }
+
+// ---------------------------------------------------------------------------
 // Batched FP64 form of the same two integrators (the plain form of the batched
 // workload): per orbit its own n_steps, dt and integrator, final state only,
 // gala's arithmetic exactly as in the kernels above.  Same work queue as the
@@ -184,6 +335,79 @@ __global__ void __launch_bounds__(128, 1) batch_fp64_kernel(const __grid_constan
     }
 }
 
+// The batch with four lanes per orbit: a CTA of four warps takes a 32-orbit block,
+// eight orbits to a warp, one CTA per SM.  For batches whose longest orbits set the
+// time rather than the FP64 pipe's throughput (few_batch_orbits): lengths 100 to
+// 2,000, MW composite, 16,384 orbits 22.0 ms one lane per orbit, 11.9 ms here; 24,000
+// 22.0 and 12.8; 40,001 22.0 and 21.2.  (Four such CTAs per SM: 25.5 ms for 16,384,
+// the longest orbits then share their scheduler from the start.)
+template <int MODE>
+__global__ void __launch_bounds__(128) batch_axis_kernel(const __grid_constant__ DevPot pot, Ruth4Coef co, int64_t n,
+                                                         int64_t slots, int32_t chunk, int64_t n_lead,
+                                                         const double *__restrict__ w0, const int64_t *__restrict__ nsteps,
+                                                         const double *__restrict__ dtv, const int32_t *__restrict__ method,
+                                                         const int32_t *__restrict__ order, int32_t *__restrict__ counter,
+                                                         double *__restrict__ out, const int32_t *__restrict__ cancel) {
+    __shared__ int64_t item;
+    __shared__ int item_sub;
+    const int lane = threadIdx.x & 31, c = lane & 3, axis = c < 2 ? c : 2;
+    const int64_t nchunks = slots / chunk;
+    const int subs = chunk / 32;
+    const AxisLane A = axis_lane(pot);
+    int phase = 0;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int sub = -1;
+            item = cancel_requested(cancel) ? -1 : queue_next_ordered(counter, nchunks, n_lead, subs, phase, sub);
+            item_sub = sub;
+        }
+        __syncthreads();
+        const int64_t ch = item;
+        const int sub = item_sub;
+        if (ch < 0) break;
+        const int b0 = sub >= 0 ? sub : 0, b1 = sub >= 0 ? sub + 1 : subs;
+        for (int b = b0; b < b1; b++) {
+            int32_t i = order[ch * chunk + 32 * b + 8 * (threadIdx.x >> 5) + (lane >> 2)];
+            // -1 pads the order; any other id outside [0, n) is skipped (and recorded once in the debug build)
+            if (i < 0 || i >= n) {
+                if (i != -1 && c == 0) (void)GX_DBG_CHECK(false, DBG_ORDER, i, n);
+                i = -1;
+            } else if (c == 0) {
+                GX_DBG_DONE(i, nsteps[i]);
+            }
+            // lanes without an orbit go along at a harmless point
+            const bool ok = i >= 0;
+            double x = ok ? w0[axis * n + i] : 1., v = ok ? w0[(3 + axis) * n + i] : 0.;
+            const double dt = ok ? dtv[i] : 0.;
+            const int64_t ns = ok ? nsteps[i] : 0;
+            auto none = [](int64_t) {};
+            // a warp's orbits are of one integrator in the schedule's orders, of both in others
+            for (int m = 0; m < 2; m++) {
+                const int64_t mine = ok && (method[i] == 0) == (m == 0) && ns > 0 ? ns : 0;
+                int64_t most = mine;
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int64_t other = __shfl_xor_sync(0xffffffffu, most, o);
+                    most = other > most ? other : most;
+                }
+                if (most == 0) continue;
+                if (m == 0) axis_run<MODE, false, false, false>(pot, A, co, dt, most, mine, axis, x, v, none);
+                else axis_run<MODE, true, false, false>(pot, A, co, dt, most, mine, axis, x, v, none);
+            }
+            if (ok && c < 3) {
+                out[axis * n + i] = x;
+                out[(3 + axis) * n + i] = v;
+            }
+        }
+    }
+}
+
+// Whether a batch is small enough for four lanes per orbit: 160 orbits per SM, where
+// the two forms meet for lengths spread 5 : 1 (26,000 orbits; for 20 : 1 it is 41,000).
+static bool few_batch_orbits(const DevPot &dp, int64_t n) {
+    return !dp.has_scf && !dp.cdev && n <= (int64_t)160 * multiprocessors();
+}
+
 static int fixed_common(const gx_potential *pot, const gx_frame *frame, const double *w0, int64_t n,
                         const double *t, int64_t ntimes, double *w_out, DevPot *dp, const char *name) {
     int rc = pack_potential(pot, dp);
@@ -211,6 +435,8 @@ int gx_leapfrog_integrate_hamiltonian(const gx_potential *pot, const gx_frame *f
     const int bs = 128;
     const unsigned grid = (unsigned)((n + bs - 1) / bs);
     cudaStream_t st = gx::as_stream(stream);
+    if (gx::few_orbits(dp, n))
+        return gx::launch_axis<false>(dp, gx::Ruth4Coef{}, w0, n, t, ntimes, save_all, w_out, st, "leapfrog");
     if (save_all && dp.has_scf)
         gx::leapfrog_kernel<true, true><<<grid, bs, 0, st>>>(dp, w0, n, t, ntimes, w_out);
     else if (save_all)
@@ -249,7 +475,17 @@ int gx_batch_integrate_fp64(const gx_potential *pot, const double *w0, int64_t n
     cudaStream_t st = gx::as_stream(stream);
     GX_CUDA_TRY(cudaMemsetAsync(queue_counter, 0, GX_BATCH_QUEUE_WORDS * sizeof(int32_t), st));
     const int64_t n_lead = gx::queue_lead_chunks(n_slots / chunk, chunk);
-    if (dp.has_scf)
+    if (gx::few_batch_orbits(dp, n)) {
+        const auto kernel = gx::axis_mode(dp) == 0   ? gx::batch_axis_kernel<0>
+                            : gx::axis_mode(dp) == 1 ? gx::batch_axis_kernel<1>
+                            : gx::axis_mode(dp) == 2 ? gx::batch_axis_kernel<2>
+                                                     : gx::batch_axis_kernel<3>;
+        // one CTA per SM, one warp per scheduler: the longest orbits, which go first, keep their pace
+        const int sms = gx::multiprocessors();
+        kernel<<<sms > 0 && sms < grid ? sms : grid, 128, 0, st>>>(dp, co, n, n_slots, chunk, n_lead, w0, n_steps, dt, method, order, queue_counter, w_out,
+                                     gx::cancel_flag());
+    }
+    else if (dp.has_scf)
         gx::batch_fp64_kernel<true><<<grid, block, 0, st>>>(dp, co, n, n_slots, chunk, n_lead, w0, n_steps, dt,
                                                             method, order, queue_counter, w_out, gx::cancel_flag());
     else
@@ -278,6 +514,7 @@ int gx_ruth4_integrate_hamiltonian(const gx_potential *pot, const gx_frame *fram
     const int bs = 128;
     const unsigned grid = (unsigned)((n + bs - 1) / bs);
     cudaStream_t st = gx::as_stream(stream);
+    if (gx::few_orbits(dp, n)) return gx::launch_axis<true>(dp, co, w0, n, t, ntimes, save_all, w_out, st, "ruth4");
     if (save_all && dp.has_scf)
         gx::ruth4_kernel<true, true><<<grid, bs, 0, st>>>(dp, co, w0, n, t, ntimes, w_out);
     else if (save_all)

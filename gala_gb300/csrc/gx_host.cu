@@ -84,8 +84,16 @@ static bool regular_component(int type, const double *P, int do_sr) {
     }
 }
 
-// Whether the packed components are a disk-bulge-halo composite; its constants.
+// Whether the packed components are a single sphere or a disk-bulge-halo composite;
+// its constants.
 static void pack_dbh(DevPot *out) {
+    if (out->ncomp == 1 && !out->c[0].do_sr &&
+        (out->c[0].type == GX_POT_HERNQUIST || out->c[0].type == GX_POT_PLUMMER)) {
+        out->sphere = out->c[0].type;
+        out->d.gm1 = out->c[0].dc[0];
+        out->d.c1 = out->c[0].type == GX_POT_PLUMMER ? out->c[0].dc[1] : out->p[out->c[0].poff + 2];
+        return;
+    }
     out->d.gm2 = 0.;
     out->d.c2 = 1.;
     int nh = 0, nd = 0, nn = 0;
@@ -104,12 +112,18 @@ static void pack_dbh(DevPot *out) {
         } else if (c.type == GX_POT_SPHERICALNFW) {
             out->d.gmh = c.dc[0];
             out->d.irs = c.dc[1];
+            out->d.vh2 = c.dc[5];
+            out->d.rs = out->p[c.poff + 2];
+            out->d.rs2 = c.dc[6];
             nn++;
         } else {
             return;
         }
     }
     out->dbh = (nh == 1 || nh == 2) && nd == 1 && nn == 1;
+    if (!out->dbh || out->c[out->ncomp - 1].type != GX_POT_SPHERICALNFW) return;
+    if (out->c[0].type == GX_POT_MIYAMOTONAGAI) out->dbh_order = 2;
+    if (out->c[out->ncomp - 2].type == GX_POT_MIYAMOTONAGAI) out->dbh_order = 1;
 }
 
 // Validate the descriptor's header and component i; *need = the doubles its type uses.

@@ -104,21 +104,17 @@ GX_HD uint64_t sqrt53(uint64_t v, uint64_t y) { return (mulhi_a(v, y) + 256) >> 
 // The same, correctly rounded: D = v 2^42 - R^2 decides (all integers; sqrt(X)
 // rounds to R exactly where -R < X - R^2 <= R).
 GX_HD uint64_t sqrt53_rn(uint64_t v, uint64_t y) {
-    uint64_t R = sqrt53(v, y);
+    const uint64_t R = sqrt53(v, y);
     const int64_t D = (int64_t)((v << 42) - R * R);
-    if (D > (int64_t)R) R++;
-    else if (D <= -(int64_t)R) R--;
-    return R;
+    return R + (uint64_t)(D > (int64_t)R) - (uint64_t)(D <= -(int64_t)R);
 }
 
 // a / b in [1, 2) for 53-bit integers with b <= a < 2 b, y = 1/b as from rcp63
 // (b taken as b 2^-52): correctly rounded to 53 bits ([2^52, 2^53]).
 GX_HD uint64_t div53_rn(uint64_t a, uint64_t b, uint64_t y) {
-    uint64_t q = (mulhi_a(a << 10, y) + 256) >> 9;  // (a 2^10)(y) >> 64 at 2^-61
+    const uint64_t q = (mulhi_a(a << 10, y) + 256) >> 9;  // (a 2^10)(y) >> 64 at 2^-61
     const int64_t r2 = (int64_t)((a << 53) - 2 * (q * b));  // twice the remainder
-    if (r2 > (int64_t)b) q++;
-    else if (r2 < -(int64_t)b) q--;
-    return q;
+    return q + (uint64_t)(r2 > (int64_t)b) - (uint64_t)(r2 < -(int64_t)b);
 }
 
 // ln m at scale 2^-64 for m in [1, 2) at scale 2^-63, c = c_j at scale 2^-32 and
@@ -151,14 +147,12 @@ GX_HD uint64_t ln_sum53(uint32_t k, uint64_t F, int &s) {
     F += b;
     F += f;
     const uint32_t ip = (uint32_t)(u2 >> 32) + (F < f ? 1u : 0u);
-    uint64_t V;  // normalised: top bit 63, value V 2^-64 2^s
-    if (ip) {
-        s = 32 - clz32(ip);
-        V = ((uint64_t)ip << (64 - s)) | (F >> s);
-    } else {
-        s = -clz64(F);
-        V = F << -s;
-    }
+    // normalised: top bit 63, value V 2^-64 2^s (both forms, one of them taken: a
+    // branch here would part the lanes of a warp)
+    const int up = 32 - clz32(ip | 1u), down = clz64(F | 1u);
+    const uint64_t Vu = ((uint64_t)ip << (64 - up)) | (F >> up), Vd = F << down;
+    const uint64_t V = ip ? Vu : Vd;
+    s = ip ? up : -down;
     return (V >> 11) + ((V >> 10) & 1u);
 }
 
@@ -204,19 +198,23 @@ __device__ __forceinline__ SqrtArg sqrt_arg(uint32_t hi, uint32_t lo) {
     const uint64_t M = ((uint64_t)m.hi << 32) | m.lo;
     const uint32_t odd = ((hi >> 20) & 1u) ^ 1u;  // biased 1023 is an even exponent
     SqrtArg a;
-    a.v = odd ? M : M >> 1;
+    a.v = M >> (1u - odd);
     a.fb = ((127u + odd) << 23) | top23(hi, lo);
     a.hbits = ((((hi >> 20) - odd + 1023u) >> 1) - 1u) << 20;  // (k' / 2 + 1022), k' = k - odd
     return a;
 }
 
+// The forms named _u take any bits and are right where ok_ says so; a straight
+// run of them leaves the compiler free to interleave their dependent chains (190
+// to 430 cycles each alone), which a branch in each would forbid.
+
 // IEEE sqrt.
-__device__ __forceinline__ double sqrt_rn(double x) {
-    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    if (!normal_pos(hi)) return sqrt(x);
-    const SqrtArg a = sqrt_arg(hi, lo);
+__device__ __forceinline__ bool ok_sqrt(double x) { return normal_pos((uint32_t)__double2hiint(x)); }
+__device__ __forceinline__ double sqrt_rn_u(double x) {
+    const SqrtArg a = sqrt_arg((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x));
     return pack53(sqrt53_rn(a.v, rsqrt63(a.v, rsqrt_seed(a.fb))), a.hbits);
 }
+__device__ __forceinline__ double sqrt_rn(double x) { return ok_sqrt(x) ? sqrt_rn_u(x) : sqrt(x); }
 // sqrt within 0.51 ulp.
 __device__ __forceinline__ double sqrt_n(double x) {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
@@ -224,12 +222,7 @@ __device__ __forceinline__ double sqrt_n(double x) {
     const SqrtArg a = sqrt_arg(hi, lo);
     return pack53(sqrt53(a.v, rsqrt63(a.v, rsqrt_seed(a.fb))), a.hbits);
 }
-// The forms named _u take any bits and are right where ok_ says so; a straight
-// run of them leaves the compiler free to interleave their dependent chains (190
-// to 430 cycles each alone), which a branch in each would forbid.
-
 // sqrt(x) (returned) and 1 / sqrt(x), each within 0.51 ulp, from one core.
-__device__ __forceinline__ bool ok_sqrt(double x) { return normal_pos((uint32_t)__double2hiint(x)); }
 __device__ __forceinline__ double sqrt_rsqrt_u(double x, double &rs) {
     const SqrtArg a = sqrt_arg((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x));
     const uint64_t y = rsqrt63(a.v, rsqrt_seed(a.fb));
@@ -259,10 +252,9 @@ __device__ __forceinline__ double rcp_u(double x) {
 }
 __device__ __forceinline__ double rcp_n(double x) { return ok_rcp(x) ? rcp_u(x) : 1.0 / x; }
 // IEEE a / b.
-__device__ __forceinline__ double div_rn(double a, double b) {
+__device__ __forceinline__ double div_rn_u(double a, double b) {
     const uint32_t ah = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
     const uint32_t bh = (uint32_t)__double2hiint(b), bl = (uint32_t)__double2loint(b);
-    if (!(mid_range(ah) & mid_range(bh))) return a / b;
     const Mant m = mant63(bh, bl);
     const uint64_t y = rcp63(m.hi, m.lo, rcp_seed(0x3f800000u | top23(bh, bl)));
     uint64_t A = ((uint64_t)(0x00100000u | (ah & 0xfffffu)) << 32) | al;
@@ -273,6 +265,8 @@ __device__ __forceinline__ double div_rn(double a, double b) {
     const uint32_t eb = (ah & 0x7ff00000u) - (bh & 0x7ff00000u) + ((1022u - less) << 20);
     return __longlong_as_double((long long)((q + ((uint64_t)eb << 32)) ^ ((uint64_t)((ah ^ bh) & 0x80000000u) << 32)));
 }
+__device__ __forceinline__ bool ok_div(double a, double b) { return ok_rcp(a) & ok_rcp(b); }
+__device__ __forceinline__ double div_rn(double a, double b) { return ok_div(a, b) ? div_rn_u(a, b) : a / b; }
 // Whether ln_n takes x: finite and at least 1 + 2^-6.
 __device__ __forceinline__ bool ln_range(double x) {
     return (uint32_t)__double2hiint(x) - 0x3ff04000u < 0x7ff00000u - 0x3ff04000u;

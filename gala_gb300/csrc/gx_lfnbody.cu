@@ -8,13 +8,19 @@ namespace gx {
 
 // ---------------------------------------------------------------------------
 // Leapfrog n-body systems: leapfrog_integrate_nbody (leapfrog.pyx:161-255) and
-// the release systems of mockstream_leapfrog (mockstream.pyx:548-593).  One
-// THREAD per system (a few bodies: the whole state fits in registers), bodies
-// updated in gala's order within a step: body k drifts, feels the external
-// potential and every other non-null massive body at its CURRENT position
-// (already moved this step when j < k: c_nbody_gradient_symplectic,
-// cpotential.cpp:418-442), and kicks.  Consecutive threads are consecutive
-// systems of one release time, so a warp runs systems of equal length.
+// the release systems of mockstream_leapfrog (mockstream.pyx:548-593).  gala moves
+// the bodies in order within a step: body k drifts, feels the external potential
+// and every other non-null massive body at its CURRENT position (already moved this
+// step when j < k: c_nbody_gradient_symplectic, cpotential.cpp:418-442), and kicks.
+// A drift depends on nothing but the body itself, so a system is a GROUP of lanes,
+// one per body: all drift, and body k takes body j's position after the drift
+// (j < k) or before it (j > k) from its lane.  The same operations in the same
+// order as one thread per system, with a step as long as one body's instead of the
+// sum over them: the kernel was bound by those chains (5 warps per SM and about 330
+// FP64 instructions per step), now by the FP64 pipe (16 warps, 115 instructions;
+// the release systems of 64 streams x 400 releases take 4.6 ms; the whole call 20.3 -> 13.0 ms).
+// Consecutive groups are consecutive systems of one release time, so a warp runs
+// systems of equal length; one-warp CTAs, longest first, fill the SMs evenly.
 // ---------------------------------------------------------------------------
 struct LfArgs {
     int64_t n_sys;
@@ -37,180 +43,134 @@ struct LfArgs {
     double t_final;
     double *stream_w_out, *nbody_w_out;
     int32_t *status;
+    int32_t gs;             // lanes per group (the largest system)
 };
 
-template <int MAXB, bool SCF>
-__device__ __forceinline__ void lf_grad(const DevPot &pot, const gx_body *__restrict__ bod, int nbody, int b,
-                                        const double (&x)[MAXB][3], double *g) {
+// Gradient at the lane's body, x after this step's drift and xo before it.  All 32
+// lanes take part: shuffles within a group's own mask would each wait on a
+// synchronisation.
+template <bool SCF>
+__device__ __forceinline__ void lf_grad(const DevPot &pot, int base, int member, bool in_sys, int nbody,
+                                        const gx_body *__restrict__ bod, const double *xo, const double *x, double *g) {
     V3 q;
-    q.v[0] = x[b][0];
-    q.v[1] = x[b][1];
-    q.v[2] = x[b][2];
+    for (int k = 0; k < 3; k++) q.v[k] = x[k];
     const V3 ge = gradient_call<SCF, true>(pot, q);
-    g[0] = ge.v[0];
-    g[1] = ge.v[1];
-    g[2] = ge.v[2];
-#pragma unroll
-    for (int j = 0; j < MAXB; j++) {
-        if (j >= nbody || j == b) continue;
+    for (int k = 0; k < 3; k++) g[k] = ge.v[k];
+    for (int j = 0; j < nbody; j++) {
+        double d[3];
+        for (int k = 0; k < 3; k++) {
+            const double xn = __shfl_sync(0xffffffffu, x[k], base + j), xp = __shfl_sync(0xffffffffu, xo[k], base + j);
+            d[k] = x[k] - (j < member ? xn : xp);
+        }
         const int type = __ldg(&bod[j].type);
-        if (type == GX_POT_NULL) continue;
-        const V3 f2 = body_gradient_call<true>(type, bod[j].params, x[b][0] - x[j][0], x[b][1] - x[j][1],
-                                         x[b][2] - x[j][2]);
-        g[0] += f2.v[0];
-        g[1] += f2.v[1];
-        g[2] += f2.v[2];
+        if (!in_sys || j == member || type == GX_POT_NULL) continue;
+        const V3 f2 = body_gradient_call<true>(type, bod[j].params, d[0], d[1], d[2]);
+        for (int k = 0; k < 3; k++) g[k] += f2.v[k];
     }
 }
 
-template <int MAXB, bool STREAM, bool SAVE_ALL, bool SCF>
-__global__ void __launch_bounds__(128) lf_nbody_kernel(const __grid_constant__ DevPot pot, const LfArgs A) {
-    const int64_t sys = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (sys >= A.n_sys) return;
-    double x[MAXB][3], v[MAXB][3], vh[MAXB][3];
-    int nsys;
-    const gx_body *bod;
-    int64_t si = 0, ss = 0, o0 = 0;
-    double t0;
-    int64_t n_steps;
+template <bool STREAM, bool SAVE_ALL, bool SCF>
+__global__ void __launch_bounds__(32) lf_nbody_kernel(const __grid_constant__ DevPot pot, const LfArgs A) {
+    const int gs = A.gs, lane = threadIdx.x;
+    const int grp = lane / gs, member = lane - grp * gs, base = grp * gs;
+    const int64_t sys = (int64_t)blockIdx.x * (32 / gs) + grp;
     const double dt = A.dt;
-    if constexpr (STREAM) {
-        si = sys / A.n_streams;
-        ss = sys - si * A.n_streams;
-        o0 = A.offset[si];
-        const int64_t o1 = A.offset[si + 1];
-        if (o1 == o0) {
-            A.status[ss * A.n_release + si] = 0;
-            return;
+    // a lane without a system or a body goes along at a harmless point
+    bool in_sys = grp < 32 / gs && sys < A.n_sys;
+    const gx_body *bod = A.bodies;
+    int64_t si = 0, ss = 0, n_steps = 0;
+    const double *src = nullptr;
+    double *o = nullptr;  // where the lane's body goes
+    int32_t *done = nullptr;
+    if (in_sys) {
+        if constexpr (STREAM) {
+            si = sys / A.n_streams;
+            ss = sys - si * A.n_streams;
+            const int64_t o0 = A.offset[si], o1 = A.offset[si + 1];
+            const bool bad = o1 < o0 || o0 < 0 || o1 > A.n_particles || A.nbody + (o1 - o0) > gs;
+            if (member == 0) {
+                done = A.status + ss * A.n_release + si;
+                if (bad) (void)GX_DBG_CHECK(!bad, DBG_OFFSET, si, A.n_release);
+                if (bad || o1 == o0) {
+                    *done = bad ? -1 : 0;
+                    done = nullptr;
+                }
+            }
+            bod = A.bodies + ss * A.nbody;
+            in_sys = !bad && o1 > o0 && member < A.nbody + (int)(o1 - o0);
+            if (in_sys) {
+                n_steps = (int64_t)((A.t_final - A.release_t[si]) / dt + 0.5);  // mockstream.pyx:582
+                if (member < A.nbody) {
+                    src = A.nbody_w + ((ss * A.n_release + si) * A.nbody + member) * 6;
+                    if (A.nbody_w_out && o1 == A.offset[A.n_release]) o = A.nbody_w_out + (ss * A.nbody + member) * 6;
+                } else {
+                    const int64_t row = ss * A.n_particles + o0 + (member - A.nbody);
+                    src = A.stream_w0 + row * 6;
+                    o = A.stream_w_out + row * 6;
+                }
+            }
+        } else {
+            bod = A.bodies + sys * A.nbody;
+            in_sys = member < A.nparticles;
+            if (in_sys) {
+                n_steps = A.ntimes - 1;
+                src = A.w0 + (sys * A.nparticles + member) * 6;
+                o = A.w_out + ((SAVE_ALL ? sys * A.ntimes : sys) * A.nparticles + member) * 6;
+            }
         }
-        if (!GX_DBG_CHECK(!(o1 < o0 || o0 < 0 || o1 > A.n_particles || A.nbody + (o1 - o0) > MAXB), DBG_OFFSET,
-                          si, A.n_release)) {
-            A.status[ss * A.n_release + si] = -1;
-            return;
-        }
-        nsys = A.nbody + (int)(o1 - o0);
-        bod = A.bodies + ss * A.nbody;
-        t0 = A.release_t[si];
-        n_steps = (int64_t)((A.t_final - t0) / dt + 0.5);  // mockstream.pyx:582
-    } else {
-        nsys = A.nparticles;
-        bod = A.bodies + sys * A.nbody;
-        t0 = A.t[0];
-        n_steps = A.ntimes - 1;
     }
-#pragma unroll
-    for (int b = 0; b < MAXB; b++) {
-        const double *src = nullptr;
-        if (b < nsys) {
-            if constexpr (STREAM)
-                src = (b < A.nbody) ? A.nbody_w + ((ss * A.n_release + si) * A.nbody + b) * 6
-                                    : A.stream_w0 + (ss * A.n_particles + o0 + (b - A.nbody)) * 6;
-            else
-                src = A.w0 + (sys * A.nparticles + b) * 6;
-        }
-#pragma unroll
+    int64_t most = n_steps;  // the warp's longest system
+    for (int k = 16; k > 0; k >>= 1) {
+        const int64_t other = __shfl_xor_sync(0xffffffffu, most, k);
+        most = other > most ? other : most;
+    }
+    double x[3], v[3], vh[3], xo[3], g[3];
+    for (int k = 0; k < 3; k++) {
+        x[k] = in_sys ? src[k] : 1.;
+        v[k] = in_sys ? src[3 + k] : 0.;
+    }
+    auto store = [&](double *p) {
         for (int k = 0; k < 3; k++) {
-            x[b][k] = src ? src[k] : 0.;
-            v[b][k] = src ? src[3 + k] : 0.;
+            p[k] = x[k];
+            p[3 + k] = v[k];
         }
-    }
-    if constexpr (!STREAM && SAVE_ALL) {
-#pragma unroll
-        for (int b = 0; b < MAXB; b++)
-            if (b < nsys) {
-                double *o = A.w_out + ((sys * A.ntimes) * A.nparticles + b) * 6;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    o[k] = x[b][k];
-                    o[3 + k] = v[b][k];
-                }
-            }
-    }
+    };
+    if (SAVE_ALL && o) store(o);
     // c_init_velocity_nbody (leapfrog.pyx:126-138), every body at the start positions
-#pragma unroll
-    for (int b = 0; b < MAXB; b++) {
-        if (b >= nsys) continue;
-        double g[3];
-        lf_grad<MAXB, SCF>(pot, bod, A.nbody, b, x, g);
-#pragma unroll
-        for (int k = 0; k < 3; k++) vh[b][k] = v[b][k] - g[k] * dt / 2.;
-    }
-    (void)t0;
-    for (int64_t j = 0; j < n_steps; j++) {
-        // c_leapfrog_step_nbody (leapfrog.pyx:140-158), bodies in order
-#pragma unroll
-        for (int b = 0; b < MAXB; b++) {
-            if (b >= nsys) continue;
-#pragma unroll
-            for (int k = 0; k < 3; k++) x[b][k] = x[b][k] + vh[b][k] * dt;
-            double g[3];
-            lf_grad<MAXB, SCF>(pot, bod, A.nbody, b, x, g);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                v[b][k] = vh[b][k] - g[k] * dt / 2.;
-                vh[b][k] = vh[b][k] - g[k] * dt;
-            }
+    lf_grad<SCF>(pot, base, member, in_sys, A.nbody, bod, x, x, g);
+    for (int k = 0; k < 3; k++) vh[k] = fma(-0.5, g[k] * dt, v[k]);  // v - g * dt / 2., the halving exact
+    for (int64_t j = 0; j < most; j++) {
+        const bool on = j < n_steps;
+        // c_leapfrog_step_nbody (leapfrog.pyx:140-158)
+        for (int k = 0; k < 3; k++) {
+            xo[k] = x[k];
+            x[k] = pick(on, x[k] + vh[k] * dt, x[k]);
         }
-        if constexpr (!STREAM && SAVE_ALL) {
-#pragma unroll
-            for (int b = 0; b < MAXB; b++)
-                if (b < nsys) {
-                    double *o = A.w_out + (((sys * A.ntimes) + j + 1) * A.nparticles + b) * 6;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        o[k] = x[b][k];
-                        o[3 + k] = v[b][k];
-                    }
-                }
+        lf_grad<SCF>(pot, base, member, in_sys, A.nbody, bod, xo, x, g);
+        for (int k = 0; k < 3; k++) {
+            const double gd = g[k] * dt;
+            if (on && (SAVE_ALL || j == n_steps - 1)) v[k] = fma(-0.5, gd, vh[k]);
+            vh[k] = pick(on, vh[k] - gd, vh[k]);
         }
+        if (SAVE_ALL && o && on) store(o + (j + 1) * A.nparticles * 6);
     }
-    if constexpr (STREAM) {
-#pragma unroll
-        for (int b = 0; b < MAXB; b++) {
-            if (b >= nsys) continue;
-            double *o;
-            if (b >= A.nbody)
-                o = A.stream_w_out + (ss * A.n_particles + o0 + (b - A.nbody)) * 6;
-            else if (A.nbody_w_out && A.offset[si + 1] == A.offset[A.n_release])
-                o = A.nbody_w_out + (ss * A.nbody + b) * 6;
-            else
-                continue;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                o[k] = x[b][k];
-                o[3 + k] = v[b][k];
-            }
-        }
-        A.status[ss * A.n_release + si] = 1;
-    } else if constexpr (!SAVE_ALL) {
-#pragma unroll
-        for (int b = 0; b < MAXB; b++)
-            if (b < nsys) {
-                double *o = A.w_out + (sys * A.nparticles + b) * 6;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    o[k] = x[b][k];
-                    o[3 + k] = v[b][k];
-                }
-            }
-    }
+    if (!SAVE_ALL && o) store(o);
+    if (STREAM && done) *done = 1;
 }
 
 template <bool STREAM, bool SAVE_ALL>
-int launch_lf(const DevPot &dp, const LfArgs &A, int maxb, cudaStream_t st) {
-    const unsigned grid = (unsigned)((A.n_sys + 127) / 128);
-    if (maxb > 8) {
-        set_error("leapfrog n-body systems of %d bodies: at most 8", maxb);
+int launch_lf(const DevPot &dp, LfArgs A, int members, cudaStream_t st) {
+    if (members > 8) {
+        set_error("leapfrog n-body systems of %d bodies: at most 8", members);
         return GX_ERR_UNSUPPORTED;
     }
-    // three bodies (a progenitor and one particle per tail) is the common mock
-    // stream; everything else up to eight bodies shares one instantiation
+    A.gs = members;
+    const int64_t per = 32 / members;
+    const unsigned grid = (unsigned)((A.n_sys + per - 1) / per);
     if (dp.has_scf)
-        lf_nbody_kernel<8, STREAM, SAVE_ALL, true><<<grid, 128, 0, st>>>(dp, A);
-    else if (maxb <= 3)
-        lf_nbody_kernel<3, STREAM, SAVE_ALL, false><<<grid, 128, 0, st>>>(dp, A);
+        lf_nbody_kernel<STREAM, SAVE_ALL, true><<<grid, 32, 0, st>>>(dp, A);
     else
-        lf_nbody_kernel<8, STREAM, SAVE_ALL, false><<<grid, 128, 0, st>>>(dp, A);
+        lf_nbody_kernel<STREAM, SAVE_ALL, false><<<grid, 32, 0, st>>>(dp, A);
     return check_launch(STREAM ? "mockstream_leapfrog" : "nbody_leapfrog");
 }
 

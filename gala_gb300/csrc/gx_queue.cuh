@@ -70,6 +70,24 @@ __device__ __forceinline__ int64_t queue_next(int32_t *queue, int64_t n_chunks, 
     return -1;
 }
 
+// The same work strictly in order -- the lead region's blocks, then the main
+// region's chunks -- for a grid whose CTAs spread a block over their four
+// schedulers; the counters mean the same.
+__device__ __forceinline__ int64_t queue_next_ordered(int32_t *queue, int64_t n_chunks, int64_t n_lead, int subs, int &phase,
+                                                      int &sub) {
+    sub = -1;
+    if (phase == 0) {
+        const int l = atomicAdd(&queue[1], 1);
+        if (l < n_lead * subs) {
+            sub = l % subs;
+            return l / subs;
+        }
+        phase = 1;
+    }
+    const int m = atomicAdd(&queue[0], 1);
+    return m < n_chunks - n_lead ? n_lead + m : -1;
+}
+
 // Host: n_lead, the lead region's chunks on the current device.
 int64_t queue_lead_chunks(int64_t n_chunks, int32_t chunk);
 
