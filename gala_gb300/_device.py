@@ -31,3 +31,30 @@ def as_device_f64(a, device=None) -> torch.Tensor:
 
 def ptr(t: torch.Tensor) -> int:
     return int(t.data_ptr())
+
+
+# Host arrays up to this many values go through one page-locked block that the
+# kernel reads and writes in place: no allocation, copy and wait on either side of
+# the launch.  Both sides of the line in the docstring below.
+STAGED_VALUES = 1 << 15
+
+
+def call_staged(name, head, a, out_size):
+    """One evaluation entry point ``name(*head, a, n, out, stream)`` on the host array
+    ``a`` (rows, n): the result's ``out_size`` values as a new numpy array.
+
+    The block comes from torch's page-locked cache and goes back to it when the
+    stream has been waited for.  Measured on a GB300, potential gradient of an MW
+    composite, device copies / in place: 257 points 95 / 50 us, 5,000 96 / 70 us,
+    10,900 96 / 88 us, 40,000 105 / 180 us."""
+    from . import _abi
+
+    size = a.size
+    block = torch.empty(size + out_size, dtype=torch.float64, pin_memory=True)
+    host = block.numpy()
+    host[:size].reshape(a.shape)[...] = a
+    p = block.data_ptr()
+    s = torch.cuda.current_stream()
+    _abi.call(name, *head, p, a.shape[1], p + 8 * size, int(s.cuda_stream))
+    s.synchronize()
+    return host[size:].copy()

@@ -192,17 +192,22 @@ class PotentialBase:
     def _eval(self, kind, q, t=0.0):
         import torch
 
-        from ._device import as_device_f64, ptr, stream_handle
+        from ._device import STAGED_VALUES, as_device_f64, call_staged, ptr, require_cuda, stream_handle
 
         q = np.asarray(q, dtype=np.float64) if not isinstance(q, torch.Tensor) else q
         shape = tuple(q.shape)
         if not shape or shape[0] != 3:  # a scalar is refused, as in gala (regression 165)
             raise ValueError(f"positions must have shape (3, ...), got {shape}")
+        name = {"value": "gx_potential_value", "gradient": "gx_potential_gradient",
+                "density": "gx_potential_density"}[kind]
+        if isinstance(q, np.ndarray) and 0 < q.size <= STAGED_VALUES:
+            require_cuda()
+            res = call_staged(name, (self.packed().for_device(), float(t)), q.reshape(3, -1),
+                              q.size if kind == "gradient" else q.size // 3)
+            return res.reshape(shape if kind == "gradient" else shape[1:])
         qd = as_device_f64(q).reshape(3, -1).contiguous()
         n = qd.shape[1]
         out = torch.empty((3, n) if kind == "gradient" else (n,), dtype=torch.float64, device=qd.device)
-        name = {"value": "gx_potential_value", "gradient": "gx_potential_gradient",
-                "density": "gx_potential_density"}[kind]
         _abi.call(name, self.packed().for_device(), float(t), ptr(qd), n, ptr(out), stream_handle())
         res = out.cpu().numpy()
         if kind == "gradient":
