@@ -30,6 +30,7 @@ UNITS = {
     "gx_host.cu": ["-fmad=false"],
     "gx_fixed.cu": ["-fmad=false"],
     "gx_dop853.cu": ["-fmad=false"],
+    "gx_dop853_axis.cu": ["-fmad=false"],
     "gx_nbody.cu": ["-fmad=false"],
     "gx_nbody_wide.cu": ["-fmad=false"],
     "gx_lfnbody.cu": ["-fmad=false"],

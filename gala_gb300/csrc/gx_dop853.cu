@@ -20,21 +20,13 @@
 //   * dense output (contd8_threadsafe, :869-904) is written directly into the
 //     (6, n_out, N) result for every requested time inside [xold, xold + h].
 // The loop is bounded by nmax like gala's; no thread ever waits on another CTA.
-#include "gx_host.h"
+#include "gx_dop853.cuh"
 #include "gx_scf.cuh"
 #include "gx_dop853_tableau.cuh"
 #include "gx_dop853_nystrom.cuh"
 #include "gx_fast64.cuh"
 
 namespace gx {
-
-struct DopArgs {
-    double atol, rtol, dt_max;
-    int64_t nmax, nstiff;
-    int64_t ntimes, out_stride, n_out;
-    int32_t save_all, nbatch;
-    const int32_t *cancel;  // host cancel flag (mapped memory) or nullptr
-};
 
 constexpr int DOP_MAX_WARPS = 32;
 
@@ -68,10 +60,6 @@ __device__ __forceinline__ void block_sum2(double &a, double &b, double *red, in
     a = sa;
     b = sb;
 }
-
-__device__ __forceinline__ double sign_d(double a, double b) { return (b < 0.0) ? -fabs(a) : fabs(a); }
-__device__ __forceinline__ double min_d(double a, double b) { return (a < b) ? a : b; }
-__device__ __forceinline__ double max_d(double a, double b) { return (a > b) ? a : b; }
 
 #define RHS(yin, kout)                                                   \
     do {                                                                 \
@@ -432,30 +420,13 @@ dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ DevFra
 // ---------------------------------------------------------------------------
 constexpr int NYS_MAX_WARPS = 8;
 
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-// 8 bytes into the shared memory of CTA `rank` of the cluster, at this CTA's address p
-__device__ __forceinline__ void cluster_store(double *p, unsigned rank, double v) {
-    unsigned a, r;
-    a = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
-}
-
 // Sums of a and b over the G warps of the batch, the same bits in every lane of
 // every warp: the two halves of a warp fold one value each, then the partial sums
 // are added in rank order.  buf: [2][NYS_MAX_WARPS], one of two used in turn.
 __device__ __forceinline__ void nys_sum2(double &a, double &b, double (*buf)[NYS_MAX_WARPS], int G, unsigned rank) {
     const int lane = threadIdx.x;
     const double oa = __shfl_xor_sync(0xffffffffu, a, 16), ob = __shfl_xor_sync(0xffffffffu, b, 16);
-    double v = lane < 16 ? a + oa : b + ob;
+    double v = pick(lane < 16, a, b) + pick(lane < 16, oa, ob);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (G == 1) {
@@ -472,12 +443,6 @@ __device__ __forceinline__ void nys_sum2(double &a, double &b, double (*buf)[NYS
         a += buf[0][k];
         b += buf[1][k];
     }
-}
-
-// The larger magnitude, by integer comparison (a double comparison is an FP64-pipe instruction).
-__device__ __forceinline__ double max_abs(double a, double b) {
-    const long long m = 0x7fffffffffffffffLL, x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
-    return __longlong_as_double(x > y ? x : y);
 }
 
 template <bool SCF>
@@ -931,6 +896,8 @@ extern "C" int gx_dop853_integrate_hamiltonian(const gx_potential *pot, const gx
     A.nbatch = nbatch;
     const int64_t nbatches = (n + nbatch - 1) / nbatch;
     cudaStream_t st = gx::as_stream(stream);
+    // Few orbits: one coordinate per lane.
+    if (gx::dop853_axis_takes(dp, df, A, n)) return gx::launch_dop853_axis(dp, df, A, w0, n, t, w_out, status, stats, st);
     // A static frame and a batch that fills one to eight warps (the portable cluster
     // size): a cluster per batch.  Several batches of at most 16 orbits stay below,
     // where two of them share a warp and with it each FP64 instruction.
