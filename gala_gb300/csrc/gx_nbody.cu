@@ -25,13 +25,20 @@
 //     compiled with -fmad=false: only the explicit fma calls fuse).
 //   * The n-body force broadcasts body j's position to the group with warp
 //     shuffles; each other lane adds -grad of body j's potential, j ascending.
-//   * The error norms and the stiffness sums are SEQUENTIAL sums in gala's
-//     component order: the running sum travels lane to lane (shuffle), each lane
-//     adding its six terms, so every norm sums in gala's order.
+//   * The error norms and the stiffness sums: each lane adds its six terms, then
+//     the members' sums are added (as a running sum from lane to lane, in gala's
+//     component order, they were 12 FP64 instructions per member and sum).
+//   * Dense output is prepared (three right-hand sides and 100 multiply-adds per
+//     component) only in a step that holds a stored time of some group of the warp;
+//     the trajectory does not use it.
+//   * Few systems go one to a warp on SMs of their own: an FP64 instruction costs a
+//     warp 64 cycles whatever its lanes do, and four warps of an SM share one unit.
+//   127 systems of 9 bodies x 300 Myr, every tenth time kept: 21.0 -> 11.5 ms with the
+//   last four points (31 ms before the force left the FP64 pipe).
 //   * Groups take systems from a global counter, longest first; a group that
 //     finishes takes the next system at once, so a warp never idles on its
 //     slowest system.  Every loop is bounded by nmax like gala's.
-#include "gx_host.h"
+#include "gx_dop853.cuh"
 #include "gx_scf.cuh"
 #include "gx_dop853_tableau.cuh"
 #include "gx_body.cuh"
@@ -41,10 +48,11 @@ static_assert(sizeof(gx_body) == 64, "gx_body layout");
 
 namespace gx {
 
-constexpr int NB_THREADS = 128;
+constexpr int NB_THREADS = 32;  // one-warp CTAs spread over the SMs
 
 struct NbArgs {
-    int32_t gs;             // lanes per group (largest system)
+    int32_t gs;             // members of the largest system
+    int32_t span;           // lanes per group
     int32_t nbody;          // massive bodies per system (the first lanes)
     int64_t n_sys;          // systems in the queue
     const gx_body *bodies;  // (n_streams or n_sys, nbody)
@@ -77,6 +85,53 @@ __device__ __forceinline__ double nb_sign(double a, double b) { return (b < 0.0)
 __device__ __forceinline__ double nb_min(double a, double b) { return (a < b) ? a : b; }
 __device__ __forceinline__ double nb_max(double a, double b) { return (a > b) ? a : b; }
 
+// A body's pull at d = (x, y, z) from it, added to k: body_gradient (gx_body.cuh) in
+// the FP64-pipe-lean forms of gx_fast64.cuh.
+__device__ __forceinline__ void body_pull(int type, const double *__restrict__ P, double x, double y, double z, double *k) {
+    const double gm = __ldg(P + 0) * __ldg(P + 1);
+    const double xy2 = fma(x, x, y * y), r2 = fma(z, z, xy2);
+    double f, fz, i;
+    switch (type) {
+    case GX_POT_KEPLER:
+        ip::sqrt_rsqrt_n(r2, i);
+        f = fz = gm * i * (i * i);
+        break;
+    case GX_POT_HERNQUIST: {
+        const double r = ip::sqrt_rsqrt_n(r2, i);
+        const double rc = fast::rcp_f(r + __ldg(P + 2));
+        f = fz = gm * i * (rc * rc);
+        break;
+    }
+    case GX_POT_PLUMMER: {
+        const double b = __ldg(P + 2);
+        ip::sqrt_rsqrt_n(fma(b, b, r2), i);
+        f = fz = gm * i * (i * i);
+        break;
+    }
+    case GX_POT_MIYAMOTONAGAI: {
+        const double a = __ldg(P + 2), b = __ldg(P + 3);
+        double isz;
+        const double zd = a + ip::sqrt_rsqrt_n(fma(z, z, b * b), isz);
+        ip::sqrt_rsqrt_n(fma(zd, zd, xy2), i);
+        f = gm * i * (i * i);
+        fz = fma(f, a * isz, f);
+        break;
+    }
+    case GX_POT_SPHERICALNFW: {
+        const double r = ip::sqrt_rsqrt_n(r2, i);
+        const double u = r * fast::rcp_f(__ldg(P + 2)), u1 = 1. + u;
+        f = fz = gm * i * (i * i) * fma(-u, fast::rcp_f(u1), fast::log_f(u1));
+        break;
+    }
+    default:  // a type without a GPU body formula poisons the result
+        f = fz = __longlong_as_double(0x7ff8000000000000LL);
+        break;
+    }
+    k[0] = fma(-f, x, k[0]);
+    k[1] = fma(-f, y, k[1]);
+    k[2] = fma(-fz, z, k[2]);
+}
+
 // Fwrapper_direct_nbody for the lane's body: Hamilton's equations in the
 // external potential, then the pull of every non-null massive body j != self.
 // Out of line (one compiled copy for the fifteen call sites of a step); the
@@ -90,13 +145,8 @@ __device__ __noinline__ V6 group_rhs_call(const DevPot &pot, const DevFrame &fr,
         const double q0y = __shfl_sync(mask, yin.v[1], base + j);
         const double q0z = __shfl_sync(mask, yin.v[2], base + j);
         const int type = __ldg(&bod[j].type);
-        if (member != j && member < nmem && type != GX_POT_NULL) {
-            double f2[3];
-            body_gradient(type, bod[j].params, yin.v[0] - q0x, yin.v[1] - q0y, yin.v[2] - q0z, f2);
-            k.v[3] += -f2[0];
-            k.v[4] += -f2[1];
-            k.v[5] += -f2[2];
-        }
+        if (member != j && member < nmem && type != GX_POT_NULL)
+            body_pull(type, bod[j].params, yin.v[0] - q0x, yin.v[1] - q0y, yin.v[2] - q0z, k.v + 3);
     }
     return k;
 }
@@ -113,24 +163,36 @@ __device__ __forceinline__ void group_rhs(const DevPot &pot, const DevFrame &fr,
     for (int c = 0; c < 6; c++) kout[c] = r.v[c];
 }
 
-// Sequential sums of two per-component series over the whole system, in gala's
-// order: lane m adds its six terms to the running sums of lanes 0..m-1.
-__device__ __forceinline__ void chain_sum2(unsigned mask, int gs, int base, int member, bool in_sys,
-                                           const double *ta, const double *tb, double &sa, double &sb) {
+// Sums of two per-component series over the whole system: each lane's six terms in
+// order, then the members' sums in order (a butterfly where the group's lanes are a
+// power of two, the lanes without a member adding zero).
+__device__ __forceinline__ void chain_sum2(unsigned mask, int gs, int span, int base, bool in_sys, const double *ta,
+                                           const double *tb, double &sa, double &sb) {
     double a = 0.0, b = 0.0;
-    for (int m = 0; m < gs; m++) {
-        if (member == m && in_sys) {
+    if (in_sys) {
+        a = ta[0];
+        b = tb[0];
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                a += ta[c];
-                b += tb[c];
-            }
+        for (int c = 1; c < 6; c++) {
+            a += ta[c];
+            b += tb[c];
         }
-        a = __shfl_sync(mask, a, base + m);
-        b = __shfl_sync(mask, b, base + m);
     }
-    sa = a;
-    sb = b;
+    if ((span & (span - 1)) == 0) {
+        for (int o = span >> 1; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(mask, a, o);
+            b += __shfl_xor_sync(mask, b, o);
+        }
+        sa = a;
+        sb = b;
+        return;
+    }
+    sa = __shfl_sync(mask, a, base);
+    sb = __shfl_sync(mask, b, base);
+    for (int m = 1; m < gs; m++) {
+        sa += __shfl_sync(mask, a, base + m);
+        sb += __shfl_sync(mask, b, base + m);
+    }
 }
 
 #define GRHS(mask_, yin_, kout_) group_rhs<SCF>(pot, fr, (mask_), base, member, nmem, A.nbody, bod, (yin_), (kout_))
@@ -141,12 +203,12 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     const __grid_constant__ NbArgs A) {
     using namespace dop;
     const int lane = threadIdx.x & 31;
-    const int gs = A.gs;
-    const int g = lane / gs;
-    const int member = lane - g * gs;
-    const int base = g * gs;
-    const bool lane_ok = g < 32 / gs;
-    const unsigned gmask = lane_ok ? (((gs == 32) ? 0xffffffffu : ((1u << gs) - 1u)) << base) : 0u;
+    const int gs = A.gs, span = A.span;
+    const int g = lane / span;
+    const int member = lane - g * span;
+    const int base = g * span;
+    const bool lane_ok = g < 32 / span;
+    const unsigned gmask = lane_ok ? (((span == 32) ? 0xffffffffu : ((1u << span) - 1u)) << base) : 0u;
 
     const double safe = 0.9, fac1 = 0.333, fac2 = 6.0;  // and beta = 0
     const double facc1 = 1.0 / fac1, facc2 = 1.0 / fac2;
@@ -157,7 +219,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
     int nmem = 0;
     const gx_body *bod = A.bodies;
     double x = 0., xend = 0., h = 0., hmax = 0., posneg = 1., uround = 0., facold = 0., hlamb = 0.;
-    int64_t nmax = 0, nstiff = 0, nfcn = 0, nstep = 0, naccpt = 0, nrejct = 0, out_idx = 0, out_slot = 0;
+    int64_t nmax = 0, nstiff = 0, nfcn = 0, nstep = 0, naccpt = 0, nrejct = 0, out_idx = 0, out_slot = 0, kept = 0;
     int last = 0, reject = 0, iasti = 0, nonsti = 0, idid = 0;
     bool have = false, done = !lane_ok, need_init = false;
 
@@ -202,7 +264,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                         for (int c = 0; c < 6; c++) y[c] = src[c];
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = 0.;
+                        for (int c = 0; c < 6; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
                     }
                     // dop853_step's dop853() arguments (dop853.pyx:46-72) and front-end defaults
                     x = A.release_t[si];
@@ -220,7 +282,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                         for (int c = 0; c < 6; c++) y[c] = src[c];
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = 0.;
+                        for (int c = 0; c < 6; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
                     }
                     // dop853_helper's dop853() arguments (dop853.pyx:157-182)
                     x = A.t[0];
@@ -240,7 +302,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 hlamb = 0.0;
                 last = reject = iasti = nonsti = idid = 0;
                 nfcn = nstep = naccpt = nrejct = 0;
-                out_idx = out_slot = 0;
+                out_idx = out_slot = kept = 0;
                 have = true;
                 need_init = true;
                 break;
@@ -268,7 +330,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                         tb[c] = sqr * sqr;
                     }
                     double dnf, dny;
-                    chain_sum2(im, gs, base, member, in_sys, ta, tb, dnf, dny);
+                    chain_sum2(im, gs, span, base, in_sys, ta, tb, dnf, dny);
                     double hh = ((dnf <= 1.0E-10) || (dny <= 1.0E-10)) ? 1.0E-6 : sqrt(dny / dnf) * 0.01;
                     hh = nb_min(hh, hmax);
                     hh = nb_sign(hh, posneg);
@@ -283,7 +345,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                         tb[c] = 0.;
                     }
                     double der2, unused;
-                    chain_sum2(im, gs, base, member, in_sys, ta, tb, der2, unused);
+                    chain_sum2(im, gs, span, base, in_sys, ta, tb, der2, unused);
                     der2 = sqrt(der2) / hh;
                     const double der12 = nb_max(fabs(der2), sqrt(dnf));
                     const double h1 =
@@ -375,7 +437,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 double t1[6], t2[6];
 #pragma unroll
                 for (int c = 0; c < 6; c++) {
-                    const double isk = fast::rcp_f(fma(rtoli, fmax(fabs(y[c]), fabs(k5[c])), atoli));
+                    const double isk = fast::rcp_f(fma(rtoli, max_abs(y[c], k5[c]), atoli));
                     double erri = fma(-bhh3, k3[c], fma(-bhh2, k9[c], fma(-bhh1, k1[c], k4[c])));
                     double sqr = erri * isk;
                     t2[c] = sqr * sqr;
@@ -384,19 +446,19 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     sqr = erri * isk;
                     t1[c] = sqr * sqr;
                 }
-                chain_sum2(am, gs, base, member, in_sys, t1, t2, err, err2);
+                chain_sum2(am, gs, span, base, in_sys, t1, t2, err, err2);
             }
-            double deno = err + 0.01 * err2;
+            double deno = fma(0.01, err2, err);
             if (deno <= 0.0) deno = 1.0;
-            err = fabs(h) * err * sqrt(1.0 / (deno * (double)(6 * nmem)));
+            err = fabs(h) * err * dsqrt(ddiv(1.0, deno * (double)(6 * nmem)));
 
             // computation of hnew (:446-452)
             // pow(err, expo1) with expo1 = 1/8 (beta = 0): three square roots
-            const double fac11 = sqrt(sqrt(sqrt(err)));
+            const double fac11 = dsqrt(dsqrt(dsqrt(err)));
             double fac = fac11;  // gala divides by pow(facold, beta) == 1 for its beta = 0
             (void)facold;
-            fac = nb_max(facc2, nb_min(facc1, fac / safe));
-            double hnew = h / fac;
+            fac = nb_max(facc2, nb_min(facc1, ddiv(fac, safe)));
+            double hnew = ddiv(h, fac);
             const bool acc = err <= 1.0;
 
             // FSAL derivative for every group; a rejected group never reads it
@@ -420,9 +482,9 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     tb[c] = sqr * sqr;
                 }
                 double stnum, stden;
-                chain_sum2(am, gs, base, member, in_sys, ta, tb, stnum, stden);
+                chain_sum2(am, gs, span, base, in_sys, ta, tb, stnum, stden);
                 if (test_st) {
-                    if (stden > 0.0) hlamb = h * sqrt(stnum / stden);
+                    if (stden > 0.0) hlamb = h * dsqrt(ddiv(stnum, stden));
                     if (hlamb > 6.1) {
                         nonsti = 0;
                         iasti++;
@@ -436,67 +498,69 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
             }
 
             if constexpr (DENSE) {
-                // dense output (:492-612), evaluated by every group, written by accepted ones
-                double r5[6], r6[6], r7[6], r8[6];
-#pragma unroll
-                for (int c = 0; c < 6; c++) {
-                    r5[c] = d41 * k1[c] + d46 * k6[c] + d47 * k7[c] + d48 * k8[c] + d49 * k9[c] + d410 * k10[c] +
-                            d411 * k2[c] + d412 * k3[c];
-                    r6[c] = d51 * k1[c] + d56 * k6[c] + d57 * k7[c] + d58 * k8[c] + d59 * k9[c] + d510 * k10[c] +
-                            d511 * k2[c] + d512 * k3[c];
-                    r7[c] = d61 * k1[c] + d66 * k6[c] + d67 * k7[c] + d68 * k8[c] + d69 * k9[c] + d610 * k10[c] +
-                            d611 * k2[c] + d612 * k3[c];
-                    r8[c] = d71 * k1[c] + d76 * k6[c] + d77 * k7[c] + d78 * k8[c] + d79 * k9[c] + d710 * k10[c] +
-                            d711 * k2[c] + d712 * k3[c];
-                }
-#pragma unroll
-                for (int c = 0; c < 6; c++)
-                    yy1[c] = fma(h, fma(a1413, k4[c], fma(a1412, k3[c], fma(a1411, k2[c], fma(a1410, k10[c],
-                        fma(a149, k9[c], fma(a148, k8[c], fma(a147, k7[c], a141 * k1[c]))))))), y[c]);
-                GRHS(am, yy1, k10);
-#pragma unroll
-                for (int c = 0; c < 6; c++)
-                    yy1[c] = fma(h, fma(a1514, k10[c], fma(a1513, k4[c], fma(a1512, k3[c], fma(a1511, k2[c],
-                        fma(a158, k8[c], fma(a157, k7[c], fma(a156, k6[c], a151 * k1[c]))))))), y[c]);
-                GRHS(am, yy1, k2);
-#pragma unroll
-                for (int c = 0; c < 6; c++)
-                    yy1[c] = fma(h, fma(a1615, k2[c], fma(a1614, k10[c], fma(a1613, k4[c], fma(a169, k9[c],
-                        fma(a168, k8[c], fma(a167, k7[c], fma(a166, k6[c], a161 * k1[c]))))))), y[c]);
-                GRHS(am, yy1, k3);
-                if (acc && !stiff) {
-                    nfcn += 3;
-                    double r1[6], r2[6], r3[6], r4[6];
-#pragma unroll
-                    for (int c = 0; c < 6; c++) {
-                        r5[c] = h * (r5[c] + d413 * k4[c] + d414 * k10[c] + d415 * k2[c] + d416 * k3[c]);
-                        r6[c] = h * (r6[c] + d513 * k4[c] + d514 * k10[c] + d515 * k2[c] + d516 * k3[c]);
-                        r7[c] = h * (r7[c] + d613 * k4[c] + d614 * k10[c] + d615 * k2[c] + d616 * k3[c]);
-                        r8[c] = h * (r8[c] + d713 * k4[c] + d714 * k10[c] + d715 * k2[c] + d716 * k3[c]);
-                        r1[c] = y[c];
-                        const double ydiff = k5[c] - y[c];
-                        r2[c] = ydiff;
-                        const double bspl = h * k1[c] - ydiff;
-                        r3[c] = bspl;
-                        r4[c] = ydiff - h * k4[c] - bspl;
-                    }
+                // dense output (:492-612): output times inside [xold, xold + hout], of which
+                // every out_stride-th is stored
+                const bool step = acc && !stiff;
+                bool store = false;
+                if (step) {
+                    nfcn += 3;  // gala prepares it on every accepted step
                     const double x0 = xold, x1 = x0 + hout;
                     while (out_idx < A.ntimes) {
                         const double t_out = A.t[out_idx];
                         if (!((x0 <= t_out && t_out <= x1) || (x1 <= t_out && t_out <= x0))) break;
-                        if (out_idx % A.out_stride == 0) {
-                            const double s = (t_out - xold) / hout;
-                            const double s1 = 1.0 - s;
-                            if (in_sys) {
-                                double *o = A.w_out + ((sys * A.n_out + out_slot) * A.nparticles + member) * 6;
-#pragma unroll
-                                for (int c = 0; c < 6; c++)
-                                    o[c] = r1[c] + s * (r2[c] + s1 * (r3[c] + s * (r4[c] +
-                                                    s1 * (r5[c] + s * (r6[c] + s1 * (r7[c] + s * r8[c]))))));
-                            }
-                            out_slot++;
-                        }
                         out_idx++;
+                    }
+                    store = kept < out_idx;
+                }
+                // prepared by every group when one needs it, written by those that do
+                if (__ballot_sync(am, store)) {
+                    double r5[6], r6[6], r7[6], r8[6];
+#define GX_D8(p)                                                                                                  \
+    fma(p##12, k3[c], fma(p##11, k2[c], fma(p##10, k10[c], fma(p##9, k9[c], fma(p##8, k8[c], fma(p##7, k7[c],      \
+        fma(p##6, k6[c], p##1 * k1[c])))))))
+#pragma unroll
+                    for (int c = 0; c < 6; c++) {
+                        r5[c] = fma(d413, k4[c], GX_D8(d4));
+                        r6[c] = fma(d513, k4[c], GX_D8(d5));
+                        r7[c] = fma(d613, k4[c], GX_D8(d6));
+                        r8[c] = fma(d713, k4[c], GX_D8(d7));
+                    }
+#undef GX_D8
+#pragma unroll
+                    for (int c = 0; c < 6; c++)
+                        yy1[c] = fma(h, fma(a1413, k4[c], fma(a1412, k3[c], fma(a1411, k2[c], fma(a1410, k10[c],
+                            fma(a149, k9[c], fma(a148, k8[c], fma(a147, k7[c], a141 * k1[c]))))))), y[c]);
+                    GRHS(am, yy1, k10);
+#pragma unroll
+                    for (int c = 0; c < 6; c++)
+                        yy1[c] = fma(h, fma(a1514, k10[c], fma(a1513, k4[c], fma(a1512, k3[c], fma(a1511, k2[c],
+                            fma(a158, k8[c], fma(a157, k7[c], fma(a156, k6[c], a151 * k1[c]))))))), y[c]);
+                    GRHS(am, yy1, k2);
+#pragma unroll
+                    for (int c = 0; c < 6; c++)
+                        yy1[c] = fma(h, fma(a1615, k2[c], fma(a1614, k10[c], fma(a1613, k4[c], fma(a169, k9[c],
+                            fma(a168, k8[c], fma(a167, k7[c], fma(a166, k6[c], a161 * k1[c]))))))), y[c]);
+                    GRHS(am, yy1, k3);
+                    if (store) {
+                        double *o = A.w_out + ((sys * A.n_out + out_slot) * A.nparticles + member) * 6;
+#pragma unroll
+                        for (int c = 0; c < 6; c++) {
+                            r5[c] = h * fma(d416, k3[c], fma(d415, k2[c], fma(d414, k10[c], r5[c])));
+                            r6[c] = h * fma(d516, k3[c], fma(d515, k2[c], fma(d514, k10[c], r6[c])));
+                            r7[c] = h * fma(d616, k3[c], fma(d615, k2[c], fma(d614, k10[c], r7[c])));
+                            r8[c] = h * fma(d716, k3[c], fma(d715, k2[c], fma(d714, k10[c], r8[c])));
+                        }
+                        for (; kept < out_idx; kept += A.out_stride, out_slot++, o += A.nparticles * 6) {
+                            const double s = ddiv(A.t[kept] - xold, hout);
+                            const double s1 = 1.0 - s;
+#pragma unroll
+                            for (int c = 0; c < 6; c++) {
+                                const double ydiff = k5[c] - y[c], bspl = fma(h, k1[c], -ydiff);
+                                const double v = fma(s, fma(s1, fma(s, fma(s1, fma(s, fma(s1, fma(s, r8[c], r7[c]), r6[c]), r5[c]),
+                                                                           fma(-h, k4[c], ydiff) - bspl), bspl), ydiff), y[c]);
+                                if (in_sys) o[c] = v;
+                            }
+                        }
                     }
                 }
             }
@@ -516,7 +580,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     reject = 0;
                 }
             } else if (!acc) {
-                hnew = h / nb_min(facc1, fac11 / safe);
+                hnew = ddiv(h, nb_min(facc1, ddiv(fac11, safe)));
                 reject = 1;
                 if (naccpt >= 1) nrejct = nrejct + 1;
                 last = 0;
@@ -719,10 +783,16 @@ __global__ void __launch_bounds__(128) fardal_sample_kernel(const __grid_constan
 }
 
 template <bool STREAM, bool DENSE>
-int launch_nbody(const DevPot &dp, const DevFrame &df, const NbArgs &A, cudaStream_t st) {
+int launch_nbody(const DevPot &dp, const DevFrame &df, NbArgs A, cudaStream_t st) {
     int dev = 0, sms = 0, per_sm = 0;
     GX_CUDA_TRY(cudaGetDevice(&dev));
     GX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // Few systems: a power of two of lanes each, as wide as leaves at most one warp per
+    // scheduler (groups of one warp that need dense output in different steps all go
+    // through it); many: the lanes they need.
+    A.span = A.gs;
+    for (int p = 1; p <= 32; p *= 2)
+        if (p >= A.gs && (A.n_sys + 32 / p - 1) / (32 / p) <= 4 * (int64_t)sms) A.span = p;
     if (dp.has_scf)
         GX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nbody_dop853_kernel<STREAM, DENSE, true>,
                                                                   NB_THREADS, 0));
@@ -730,7 +800,7 @@ int launch_nbody(const DevPot &dp, const DevFrame &df, const NbArgs &A, cudaStre
         GX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nbody_dop853_kernel<STREAM, DENSE, false>,
                                                                   NB_THREADS, 0));
     if (per_sm < 1) per_sm = 1;
-    const int64_t groups_per_block = (int64_t)(NB_THREADS / 32) * (32 / A.gs);
+    const int64_t groups_per_block = (int64_t)(NB_THREADS / 32) * (32 / A.span);
     int64_t need = (A.n_sys + groups_per_block - 1) / groups_per_block;
     int64_t grid = (int64_t)sms * per_sm;
     if (need < grid) grid = need;
