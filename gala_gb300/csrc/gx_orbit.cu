@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "gx_host.h"
+#include "gx_ipipe.cuh"
 
 namespace gx {
 
@@ -23,10 +24,8 @@ struct ExtArgs {
     const double *w;   // (6, ntimes, n)
     const double *t;   // (ntimes)
     int64_t ntimes, n;
-    int32_t reverse;   // time grid runs backwards: scan from the end (gala reverses the orbit)
     int32_t approximate;
     int32_t keep;
-    int32_t pad;
     int32_t *count;    // (3, n)
     double *sum, *vmin, *vmax;  // (3, n)
     double *vals, *times;       // (3, n, keep) or NULL
@@ -66,6 +65,7 @@ __device__ __forceinline__ void ext_push(const ExtArgs &A, ExtAcc &acc, int kind
 // D = s0 s2 (s2 - s0), q = q1 + (B s + C s^2) / D where C = e2 s0 - e0 s2 and
 // B = e2 s0 (s2 - s0) - C s2; the vertex is at s = -B / (2C), value
 // q1 - B^2 / (4 C D).  One reciprocal instead of gala's polyfit.
+template <bool TIMES>
 __device__ __forceinline__ void vertex(double q0, double q1, double q2, double t0, double t1, double t2, double &v,
                                        double &tv) {
     const double s0 = t0 - t1, s2 = t2 - t1, w = s2 - s0;
@@ -73,8 +73,8 @@ __device__ __forceinline__ void vertex(double q0, double q1, double q2, double t
     const double C = fma(e2, s0, -e0 * s2);
     const double B = fma(e2 * s0, w, -C * s2);
     const double D = s0 * s2 * w;
-    const double inv = 1.0 / (2.0 * C * D);
-    tv = t1 - B * D * inv;
+    const double inv = ip::rcp_n(2.0 * C * D);
+    if (TIMES) tv = t1 - B * D * inv;
     v = q1 - 0.5 * B * B * inv;
 }
 
@@ -95,7 +95,7 @@ __device__ __forceinline__ void vertex(double q0, double q1, double q2, double t
 // candidates were staged.  Pericentre and apocentre share the parabola of r:
 // the vertex of -r is minus the vertex of r, bit for bit.
 constexpr int EXT_U = 2;        // samples per chunk
-constexpr int EXT_STAGES = 2;   // chunks in shared memory: one being scanned, one in flight
+constexpr int EXT_STAGES = 3;   // chunks in shared memory: one being scanned, the others in flight (2, 3, 4: 222, 217, 259 us)
 static_assert(EXT_U >= 2, "the window carries two samples out of each chunk");
 constexpr int EXT_CAP = 64;     // ring slots per warp and kind
 constexpr int EXT_WARPS = 8;    // warps per CTA (time segments per orbit group)
@@ -129,46 +129,26 @@ struct ExtRings {
     int znext[EXT_CAP];
 };
 
-// sqrt(u) for u >= 0 from an FP32 reciprocal-square-root seed and STEPS Newton
-// (Heron) steps in FP64: relative error below 1e-13 after one step (the seed's
-// ~3e-7, squared), a few ulp after two; three FP64 instructions a step instead
-// of a correctly rounded square root.
-template <int STEPS>
-__device__ __forceinline__ double sqrt_newton(double u) {
-    const unsigned hi = (unsigned)__double2hiint(u);
-    if (hi < (897u << 20) || hi >= (1151u << 20)) return sqrt(u);  // outside the FP32 normal range
-    const unsigned lo = (unsigned)__double2loint(u);
-    const float uf = __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
-    const unsigned yb = __float_as_uint(rsqrtf(uf));
-    // the FP32 seed as a double, and half of it, built from its bits
-    const int yhi = (int)(((yb >> 23) + 896u) << 20 | ((yb >> 3) & 0xfffffu));
-    const int ylo = (int)(yb << 29);
-    const double y = __hiloint2double(yhi, ylo), h = __hiloint2double(yhi - (1 << 20), ylo);
-    double r = u * y;
-#pragma unroll
-    for (int k = 0; k < STEPS; k++) r = fma(fma(-r, r, u), h, r);
-    return r;
-}
-
 // The vertex of the parabola through (t_k, r_k), r_k = sqrt(u_k), as vertex()
 // computes it, with the differences r_k - r_1 taken as (u_k - u_1) / (r_k + r_1):
-// exact up to the rounding of u, so the square roots (from sqrt_newton) only
-// need the accuracy of a ratio.  With a_k = r_k + r_1 and P = a_0 a_2 the
+// exact up to the rounding of u.  With a_k = r_k + r_1 and P = a_0 a_2 the
 // centred coefficients are C' / P and B' / P (C' and B' as in vertex() with
 // e_0 a_0 a_2 = (u_0 - u_1) a_2 and e_2 a_0 a_2 = (u_2 - u_1) a_0); P cancels in
-// the vertex position and one reciprocal serves both outputs.
+// the vertex position and one reciprocal serves both outputs.  Square roots and
+// reciprocals run on the integer pipe (gx_ipipe.cuh): the checks' FP64 instructions,
+// not the scan's bytes, are what bounds populations with many extrema.
+template <bool TIMES>
 __device__ __forceinline__ void vertex_r(double u0, double u1, double u2, double t0, double t1, double t2,
                                          double &v, double &tv) {
-    // r_0, r_2 enter only through the ratios; r_1 is the value's leading term
-    const double r0 = sqrt_newton<1>(u0), r1 = sqrt_newton<2>(u1), r2 = sqrt_newton<1>(u2);
+    const double r0 = ip::sqrt_n(u0), r1 = ip::sqrt_n(u1), r2 = ip::sqrt_n(u2);
     const double s0 = t0 - t1, s2 = t2 - t1, w = s2 - s0;
     const double a0 = r0 + r1, a2 = r2 + r1;
     const double p0 = (u0 - u1) * a2, p2 = (u2 - u1) * a0;  // e_k a_0 a_2
     const double C = fma(p2, s0, -p0 * s2);
     const double B = fma(p2 * s0, w, -C * s2);
     const double DP = (s0 * s2 * w) * (a0 * a2);
-    const double inv = 1.0 / (2.0 * C * DP);
-    tv = t1 - B * DP * inv;
+    const double inv = ip::rcp_n(2.0 * C * DP);
+    if (TIMES) tv = t1 - B * DP * inv;
     v = r1 - 0.5 * B * B * inv;
 }
 
@@ -183,10 +163,11 @@ constexpr long long EXT_INF_BITS = 0x7ff0000000000000LL;
 // (orbit.py:405, argrelmax) are made on r^2 and |z| as integers (FP64
 // comparisons cost a slot of the FP64 pipe); a NaN sample is never an extremum
 // and has none next to it, as in argrelmax.
-__device__ __noinline__ void ext_flush(const ExtArgs &A, ExtRings &R, ExtAcc *acc, int64_t i, int lane, int nr,
-                                       int nz, int rhead, int zhead) {
+template <bool TIMES>  // the times of the extrema are wanted
+__device__ __noinline__ void ext_flush(const ExtArgs &A, bool reverse, ExtRings &R, ExtAcc *acc, int64_t i, int lane,
+                                       int nr, int nz, int rhead, int zhead) {
     const int nt = (int)A.ntimes;
-    auto tval = [&](int j) { return __ldg(A.t + (A.reverse ? nt - 1 - j : j)); };
+    auto tval = [&](int j) { return __ldg(A.t + (reverse ? nt - 1 - j : j)); };
     __syncwarp();
     for (int s = lane; s < nr; s += 32) {
         double u[3];
@@ -208,9 +189,9 @@ __device__ __noinline__ void ext_flush(const ExtArgs &A, ExtRings &R, ExtAcc *ac
             if (A.approximate)
                 v = sqrt(u[1]);
             else
-                vertex_r(u[0], u[1], u[2], tval(j - 1), t1, tval(j + 1), v, tv);
+                vertex_r<TIMES>(u[0], u[1], u[2], tval(j - 1), t1, tval(j + 1), v, tv);
             R.r[0][s] = v;
-            R.r[1][s] = tv;
+            if (TIMES) R.r[1][s] = tv;
         }
         R.rj[s] = kind;
     }
@@ -226,10 +207,10 @@ __device__ __noinline__ void ext_flush(const ExtArgs &A, ExtRings &R, ExtAcc *ac
             const double t1 = tval(j);
             double v = a1, tv = t1;
             if (!A.approximate)
-                vertex(__longlong_as_double(k0), a1, __longlong_as_double(k2), tval(j - 1), t1, tval(j + 1), v,
+                vertex<TIMES>(__longlong_as_double(k0), a1, __longlong_as_double(k2), tval(j - 1), t1, tval(j + 1), v,
                        tv);
             R.z[0][s] = v;
-            R.z[1][s] = tv;
+            if (TIMES) R.z[1][s] = tv;
         }
         R.zj[s] = kind;
     }
@@ -274,19 +255,23 @@ __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_oldest() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(EXT_STAGES - 1) : "memory");
+}
 
-// Scan samples [js, je) of orbit ii (scan order) and fold the extrema centred
+// Scan samples [js, je) of orbit ii (scan order: from the last sample where the time
+// grid runs backwards, as gala reverses the orbit) and fold the extrema centred
 // in [clo, chi) into acc.  All lanes of the warp call it together.
-__device__ __forceinline__ void ext_scan(const ExtArgs &A, ExtWarp &Wp, ExtAcc *acc, int64_t ii, bool live, int js,
-                                         int je, int clo, int chi) {
+template <bool TIMES>
+__device__ __forceinline__ void ext_scan(const ExtArgs &A, bool reverse, ExtWarp &Wp, ExtAcc *acc, int64_t ii, bool live,
+                                         int js, int je, int clo, int chi) {
     ExtRings &R = Wp.rings;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const int64_t nt = A.ntimes;
     // sample j of the scan is row (reverse ? nt-1-j : j); rows are n doubles apart
-    const int64_t step = A.reverse ? -A.n : A.n;
-    const double *p0 = A.w + ii + (A.reverse ? (nt - 1) * A.n : 0) + js * step;
+    const int64_t step = reverse ? -A.n : A.n;
+    const double *p0 = A.w + ii + (reverse ? (nt - 1) * A.n : 0) + js * step;
     const int64_t plane = nt * A.n;  // x -> y -> z
     int nr = 0, nz = 0;                                  // ring fill (warp-uniform)
     int rhead = -1, rlast = -1, zhead = -1, zlast = -1;  // this lane's chains
@@ -299,7 +284,7 @@ __device__ __forceinline__ void ext_scan(const ExtArgs &A, ExtWarp &Wp, ExtAcc *
         const unsigned br = __ballot_sync(0xffffffffu, vr), bz = __ballot_sync(0xffffffffu, vz);
         if ((br | bz) == 0u) return;
         if (nr + __popc(br) > EXT_CAP || nz + __popc(bz) > EXT_CAP) {
-            ext_flush(A, R, acc, ii, lane, nr, nz, rhead, zhead);
+            ext_flush<TIMES>(A, reverse, R, acc, ii, lane, nr, nz, rhead, zhead);
             nr = nz = 0;
             rhead = rlast = zhead = zlast = -1;
         }
@@ -345,12 +330,14 @@ __device__ __forceinline__ void ext_scan(const ExtArgs &A, ExtWarp &Wp, ExtAcc *
     bool znz[EXT_U + 2];
     wr[0] = wr[1] = wa[0] = wa[1] = 0.f;
     znz[0] = znz[1] = false;
-    if (nchunk > 0) issue(0);
-    cp_async_commit();
-    for (int k = 0; k < nchunk; k++) {
-        if (k + 1 < nchunk) issue(k + 1);
+    for (int k = 0; k < EXT_STAGES - 1; k++) {
+        if (k < nchunk) issue(k);
         cp_async_commit();
-        cp_async_wait_prev();  // this lane's copies of chunk k have landed
+    }
+    for (int k = 0; k < nchunk; k++) {
+        if (k + EXT_STAGES - 1 < nchunk) issue(k + EXT_STAGES - 1);
+        cp_async_commit();
+        cp_async_wait_oldest();  // this lane's copies of chunk k have landed
         const double(*b)[EXT_U][32] = Wp.buf[k % EXT_STAGES];
 #pragma unroll
         for (int u = 0; u < EXT_U; u++) {
@@ -392,7 +379,7 @@ __device__ __forceinline__ void ext_scan(const ExtArgs &A, ExtWarp &Wp, ExtAcc *
         cx0 = cx1; cy0 = cy1; cz0 = cz1; wr[0] = wr[1]; wa[0] = wa[1];
         cx1 = x; cy1 = y; cz1 = z; wr[1] = wr[2]; wa[1] = wa[2];
     }
-    ext_flush(A, R, acc, ii, lane, nr, nz, rhead, zhead);
+    ext_flush<TIMES>(A, reverse, R, acc, ii, lane, nr, nz, rhead, zhead);
 }
 
 __device__ __forceinline__ void ext_reset(ExtAcc *acc) {
@@ -414,32 +401,52 @@ __device__ __forceinline__ void ext_store(const ExtArgs &A, int k, int64_t i, in
     A.vmax[k * A.n + i] = count ? from_key(kmax) : nan;
 }
 
-// Persistent CTAs of EXT_WARPS warps over groups of 32 orbits (one orbit per
-// lane).  Statistics only (keep = 0): the CTA's warps split one group's time
-// range into EXT_WARPS segments and the partial statistics are merged in
-// shared memory in segment (time) order, so every SM stays busy to the end
-// whatever N is.  With keep > 0 (the first extrema themselves, in time order)
-// each warp scans a whole group.
-__global__ void __launch_bounds__(EXT_THREADS, 2) orbit_extrema_kernel(const ExtArgs A) {
+// 16 bytes of partial statistics of another CTA of the cluster: the same shared
+// address in CTA `rank`.
+__device__ __forceinline__ const ExtPart *ext_remote(const ExtPart *p, unsigned rank) {
+    unsigned long long r;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+    return reinterpret_cast<const ExtPart *>(r);
+}
+__device__ __forceinline__ void ext_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Persistent CTAs of EXT_WARPS warps over groups [g0, g1) of 32 orbits (one orbit per
+// lane).  Statistics only (keep = 0): the warps split one group's time range into
+// segments and the partial statistics are merged in segment (time) order.  Segments
+// are long (a segment's pipeline fill and last candidates are a few microseconds
+// of latency), so whole rounds over the groups take one CTA per group; the groups left
+// over for a last round that would be mostly idle are split further, over a cluster of
+// up to 8 CTAs each, whose first merges.  626 groups x 1,001 samples: 226 -> 195 us
+// with that and the checks' roots and reciprocals off the FP64 pipe.
+// With keep > 0 (the first extrema themselves, in time order) each warp scans a whole
+// group and a cluster is one CTA.
+__global__ void __launch_bounds__(EXT_THREADS, 2) orbit_extrema_kernel(const ExtArgs A, int64_t g0, int64_t g1,
+                                                                        int cluster) {
     extern __shared__ __align__(16) unsigned char ext_smem[];
     ExtWarp *warps = reinterpret_cast<ExtWarp *>(ext_smem);  // [EXT_WARPS]
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ExtWarp &Wp = warps[wid];
     const int nt = (int)A.ntimes;
+    const bool reverse = nt >= 2 && __ldg(A.t + nt - 1) < __ldg(A.t);
     const int64_t ngroups = (A.n + 31) / 32;
     const bool split = A.vals == nullptr;
-    const int64_t units = split ? ngroups : (ngroups + EXT_WARPS - 1) / EXT_WARPS;
+    const int64_t units = split ? g1 - g0 : (ngroups + EXT_WARPS - 1) / EXT_WARPS;
+    const int rank = blockIdx.x % cluster, segs = cluster * EXT_WARPS;
     ExtAcc acc[3];
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int64_t g = split ? u : u * EXT_WARPS + wid;
+    for (int64_t u = blockIdx.x / cluster; u < units; u += gridDim.x / cluster) {
+        const int64_t g = split ? g0 + u : u * EXT_WARPS + wid;
         const int64_t i = g * 32 + lane;
         const bool live = g < ngroups && i < A.n;
         const int64_t ii = live ? i : 0;
         ext_reset(acc);
         if (split) {
-            const int seg = (nt + EXT_WARPS - 1) / EXT_WARPS;
-            const int lo = wid * seg, hi = min(nt, lo + seg);
-            if (lo < hi) ext_scan(A, Wp, acc, ii, live, max(lo - 1, 0), min(hi + 1, nt), max(lo, 1), min(hi, nt - 1));
+            const int seg = (nt + segs - 1) / segs;
+            const int lo = min((rank * EXT_WARPS + wid) * seg, nt), hi = min(nt, lo + seg);
+            if (lo < hi)
+                ext_scan<false>(A, reverse, Wp, acc, ii, live, max(lo - 1, 0), min(hi + 1, nt), max(lo, 1), min(hi, nt - 1));
             ExtPart &P = *reinterpret_cast<ExtPart *>(&Wp.rings.r[0][0]);
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -448,31 +455,50 @@ __global__ void __launch_bounds__(EXT_THREADS, 2) orbit_extrema_kernel(const Ext
                 P.kmin[k][lane] = acc[k].kmin;
                 P.kmax[k][lane] = acc[k].kmax;
             }
-            __syncthreads();
-            if (threadIdx.x < 96) {
+            if (cluster > 1) ext_cluster_sync();
+            else __syncthreads();
+            if (rank == 0 && threadIdx.x < 96) {
                 const int k = threadIdx.x >> 5;
                 const int64_t io = g * 32 + lane;
                 int32_t count = 0;
                 double sum = 0.;
                 long long kmin = 0x7fffffffffffffffLL, kmax = -0x7fffffffffffffffLL - 1;
-                for (int w = 0; w < EXT_WARPS; w++) {
-                    const ExtPart &Q = *reinterpret_cast<const ExtPart *>(&warps[w].rings.r[0][0]);
-                    if (Q.count[k][lane] == 0) continue;
-                    count += Q.count[k][lane];
-                    sum += Q.sum[k][lane];
-                    kmin = min(kmin, Q.kmin[k][lane]);
-                    kmax = max(kmax, Q.kmax[k][lane]);
+                for (int w = 0; w < segs; w++) {
+                    const ExtPart *Q = reinterpret_cast<const ExtPart *>(&warps[w % EXT_WARPS].rings.r[0][0]);
+                    if (w >= EXT_WARPS) Q = ext_remote(Q, w / EXT_WARPS);
+                    if (Q->count[k][lane] == 0) continue;
+                    count += Q->count[k][lane];
+                    sum += Q->sum[k][lane];
+                    kmin = min(kmin, Q->kmin[k][lane]);
+                    kmax = max(kmax, Q->kmax[k][lane]);
                 }
                 if (io < A.n) ext_store(A, k, io, count, sum, kmin, kmax);
             }
-            __syncthreads();
+            if (cluster > 1) ext_cluster_sync();
+            else __syncthreads();
         } else if (g < ngroups) {
-            ext_scan(A, Wp, acc, ii, live, 0, nt, 1, nt - 1);
+            ext_scan<true>(A, reverse, Wp, acc, ii, live, 0, nt, 1, nt - 1);
             if (live)
 #pragma unroll
                 for (int k = 0; k < 3; k++) ext_store(A, k, i, acc[k].count, acc[k].sum, acc[k].kmin, acc[k].kmax);
         }
     }
+}
+
+static cudaError_t launch_extrema(const ExtArgs &A, int64_t g0, int64_t g1, int cluster, unsigned grid, size_t smem,
+                                  cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(EXT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, orbit_extrema_kernel, A, g0, g1, cluster);
 }
 
 }  // namespace gx
@@ -493,22 +519,12 @@ extern "C" int gx_orbit_extrema(const double *w, const double *t, int64_t ntimes
     A.n = n;
     A.approximate = approximate ? 1 : 0;
     A.keep = keep;
-    A.pad = 0;
     A.count = count;
     A.sum = sum;
     A.vmin = vmin;
     A.vmax = vmax;
     A.vals = keep ? vals : nullptr;
     A.times = keep ? times : nullptr;
-    A.reverse = 0;
-    if (ntimes >= 2) {
-        double tt[2];
-        cudaStream_t st = gx::as_stream(stream);
-        GX_CUDA_TRY(cudaMemcpyAsync(&tt[0], t, sizeof(double), cudaMemcpyDeviceToHost, st));
-        GX_CUDA_TRY(cudaMemcpyAsync(&tt[1], t + ntimes - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
-        GX_CUDA_TRY(cudaStreamSynchronize(st));
-        A.reverse = tt[1] < tt[0] ? 1 : 0;
-    }
     int dev = 0, sms = 0, per_sm = 0;
     const size_t smem = sizeof(gx::ExtWarp) * gx::EXT_WARPS;
     GX_CUDA_TRY(cudaGetDevice(&dev));
@@ -518,8 +534,18 @@ extern "C" int gx_orbit_extrema(const double *w, const double *t, int64_t ntimes
     GX_CUDA_TRY(
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gx::orbit_extrema_kernel, gx::EXT_THREADS, smem));
     const int64_t groups = (n + 31) / 32;
-    const int64_t units = keep ? (groups + gx::EXT_WARPS - 1) / gx::EXT_WARPS : groups;
-    const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)sms * std::max(per_sm, 1));
-    gx::orbit_extrema_kernel<<<grid, gx::EXT_THREADS, smem, gx::as_stream(stream)>>>(A);
+    const int64_t slots = (int64_t)sms * std::max(per_sm, 1);
+    cudaStream_t st = gx::as_stream(stream);
+    if (keep) {
+        const int64_t units = (groups + gx::EXT_WARPS - 1) / gx::EXT_WARPS;
+        GX_CUDA_TRY(gx::launch_extrema(A, 0, groups, 1, (unsigned)std::min(units, slots), smem, st));
+        return gx::check_launch("orbit_extrema");
+    }
+    // whole rounds, then what is left over
+    const int64_t whole = groups / slots * slots, rest = groups - whole;
+    if (whole) GX_CUDA_TRY(gx::launch_extrema(A, 0, whole, 1, (unsigned)slots, smem, st));
+    int cluster = 1;
+    while (cluster < 8 && rest * cluster * 2 <= slots) cluster *= 2;
+    if (rest) GX_CUDA_TRY(gx::launch_extrema(A, whole, groups, cluster, (unsigned)(rest * cluster), smem, st));
     return gx::check_launch("orbit_extrema");
 }

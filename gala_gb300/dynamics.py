@@ -551,15 +551,22 @@ class Orbit(PhaseSpacePosition):
         wd, td = self._device_w_t()
         nt, n = int(wd.shape[1]), int(wd.shape[2])
         dev = wd.device
-        count = torch.zeros((3, n), dtype=torch.int32, device=dev)
-        sm, mn, mx = (torch.zeros((3, n), dtype=torch.float64, device=dev) for _ in range(3))
+        # sums, minima, maxima and counts in one block, written whole by the kernel and
+        # brought back in one copy
+        stats = torch.empty(9 * n + (3 * n + 1) // 2, dtype=torch.float64, device=dev)
+        sm, mn, mx = (stats[3 * n * k:3 * n * (k + 1)] for k in range(3))
+        count = stats[9 * n:]
         vals = torch.zeros((3, n, keep), dtype=torch.float64, device=dev) if keep else None
         times = torch.zeros((3, n, keep), dtype=torch.float64, device=dev) if keep else None
         _abi.call("gx_orbit_extrema", ptr(wd), ptr(td), nt, n, int(bool(approximate)), int(keep), ptr(count),
                   ptr(sm), ptr(mn), ptr(mx), ptr(vals) if keep else None, ptr(times) if keep else None,
                   stream_handle())
-        out = {"count": count.cpu().numpy(), "sum": sm.cpu().numpy(), "min": mn.cpu().numpy(),
-               "max": mx.cpu().numpy()}
+        host = torch.empty(stats.shape, dtype=stats.dtype, pin_memory=True)
+        host.copy_(stats, non_blocking=True)
+        torch.cuda.current_stream().synchronize()
+        host = host.numpy()
+        out = {k: host[3 * n * i:3 * n * (i + 1)].reshape(3, n) for i, k in enumerate(("sum", "min", "max"))}
+        out["count"] = host[9 * n:].view(np.int32)[:3 * n].reshape(3, n)
         if keep:
             out["vals"] = vals.cpu().numpy()
             out["times"] = times.cpu().numpy()
