@@ -15,132 +15,376 @@
 //                forward pass (Zbar_4 += e w5 * S_4, W_l g += Zbar_l^T A_{l-1},
 //                Abar = Zbar_l W_l, Zbar_{l-1} += Abar * S_{l-1}).
 // Parameter gradients are written to `grads`; gx_mlp_adam applies Adam.
-// Every GEMM is one tiled SIMT kernel (64x64 tiles, 4x4 outputs per thread).
+// Every 256-wide product is a tiled FP32 kernel (rows_kernel, with the elementwise pass
+// that follows it in its epilogue; grads_kernel for the weights); the products with the
+// 3-wide input or gradient are row and column reductions of their own.  What bounds a
+// step is the FP32 pipe: 18 products of batch x 256 x 256.  Batch 8,192, 16 steps: 21.1 -> 12.6 ms.
 #include "gx_host.h"
 #include "gx_mlp.cuh"
 
 namespace gx {
 namespace mlp {
 
-// C[M,N] = alpha * op(A)[M,K] op(B)[K,N] + beta * C.  TA: A is stored [K][M]
-// (element (m,k) at A[k*lda+m]) instead of [M][K]; TB: B stored [N][K].
-// 128 x 128 block tile, K slabs of 8 staged through shared memory (double
-// buffered), 256 threads each computing an 8 x 8 register tile.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) gemm_f32(int M, int N, int K, float alpha, const float *__restrict__ A,
-                                                int lda, const float *__restrict__ B, int ldb, float beta,
-                                                float *__restrict__ C, int ldc) {
-    constexpr int BM = 128, BN = 128, BK = 8;
-    __shared__ __align__(16) float As[2][BK][BM];
-    __shared__ __align__(16) float Bs[2][BK][BN];
+// What happens to a product d on its way out:
+//   EPI_ACT   z = d + bias -> C = silu(z), p = silu'(z), q = silu''(z)
+//   EPI_UD    C = d, p = d * S
+//   EPI_ADJ   C = d * S, p = d * U * T
+//   EPI_LAST  C = d * S, p = bias (d * T + e S)            (bias the output weights, e per row)
+//   EPI_MAC   C += d * S
+enum { EPI_ACT, EPI_UD, EPI_ADJ, EPI_LAST, EPI_MAC };
+
+static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+
+struct Epi {
+    const float *bias, *S, *U, *T, *e;
+    float *p, *q;
+};
+
+// two FP32 multiply-adds (each rounded as fmaf) in one instruction
+__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t twice(float x) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 halves(uint64_t x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+// four floats into shared memory (zeros unless `in`); VEC: both addresses are multiples of 16 bytes
+template <bool VEC>
+__device__ __forceinline__ void copy4(float *dst, const float *src, bool in) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * i), "l"(src + i), "r"(in ? 4 : 0)
+                         : "memory");
+    }
+}
+__device__ __forceinline__ void copies_end() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copies_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float *p) {
+    if (VEC) return *reinterpret_cast<const float4 *>(p);
+    return make_float4(p[0], p[1], p[2], p[3]);
+}
+template <bool VEC>
+__device__ __forceinline__ void store4(float *p, float4 v) {
+    if (VEC) {
+        *reinterpret_cast<float4 *>(p) = v;
+    } else {
+        p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+    }
+}
+__device__ __forceinline__ float4 operator*(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+
+// Both products run 128 x 64 tiles, 256 threads of 8 x 4 outputs, two CTAs per SM, over
+// K slabs of 16 held [k][row] and [k][column] in three stages of shared memory.  A slab
+// is a thousand cycles of the FP32 pipe, about a read that misses L2, so two of them are
+// in flight (one slab ahead, 128 x 128 tiles and one CTA per SM left the FP32 pipe 60%
+// idle, half of that waiting for global memory).  One instruction multiplies two
+// neighbouring rows; with two neighbouring k instead, which needs no transposing, there
+// were not the registers to read ahead and rows_kernel took 39 to 60 us for 34 to 38.
+constexpr int BM = 128, BN = 64, BK = 16, STAGES = 3;
+constexpr int LDM = BM + 4, LDN = BN + 4;
+typedef float SlabA[BK][LDM];
+typedef float SlabB[BK][LDN];
+
+__device__ __forceinline__ void slab_product(uint64_t (&acc)[4][4], const SlabA &As, const SlabB &Bs, int tx, int ty) {
+#pragma unroll
+    for (int kk = 0; kk < BK; kk++) {
+        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(&As[kk][ty * 4]);
+        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(&As[kk][64 + ty * 4]);
+        const float4 bv = *reinterpret_cast<const float4 *>(&Bs[kk][tx * 4]);
+        const uint64_t a[4] = {a0.x, a0.y, a1.x, a1.y};
+        const uint64_t b[4] = {twice(bv.x), twice(bv.y), twice(bv.z), twice(bv.w)};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) fma2(acc[i][j], a[i], b[j]);
+    }
+}
+// the tile's row of acc[i], half r, and its four values
+__device__ __forceinline__ int tile_row(int i, int r, int ty) { return (i < 2 ? 0 : 60) + ty * 4 + 2 * i + r; }
+__device__ __forceinline__ float4 tile_values(const uint64_t (&c)[4], int r) {
+    const float2 v0 = halves(c[0]), v1 = halves(c[1]), v2 = halves(c[2]), v3 = halves(c[3]);
+    return r ? make_float4(v0.y, v1.y, v2.y, v3.y) : make_float4(v0.x, v1.x, v2.x, v3.x);
+}
+
+// C[M,H] = A[M,H] op(W) and the epilogue; A and C are [M][H], W is [n][k] with TB, else
+// [k][n].  What is stored k-contiguous passes through registers and is transposed on the
+// way to shared memory (two lanes to a row of 8 k, 4 LDM = 4 LDN = 16 mod 32: no bank
+// conflicts), the rest is copied there.
+// 8,192 x 256 x 256: 38 -> 34 to 38 us, with the elementwise pass that followed
+// it (8-9 us) inside.
+template <bool TB, int EPI, bool VEC>
+__global__ void __launch_bounds__(256, 2) rows_kernel(int M, const float *__restrict__ A, const float *__restrict__ W,
+                                                      float *C, Epi ep) {
+    constexpr int SLABS = H / BK;
+    __shared__ __align__(16) SlabA As[STAGES];
+    __shared__ __align__(16) SlabB Bs[STAGES];
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    // split-K: this CTA covers K range [kbeg, kend)
-    const int kchunk = ((K + gridDim.z - 1) / gridDim.z + BK - 1) / BK * BK;
-    const int kbeg = blockIdx.z * kchunk;
-    const int kend = min(K, kbeg + kchunk);
-    float acc[8][8] = {};
-    float ra[4], rb[4];
-    auto gload = [&](int k0) {
+    // what this thread brings in: rows `row` and row + 64, four k from kq
+    const int kq = (tid % 2 + 2 * (tid / 128)) * 4, row = tid % 128 / 2;
+    float4 ra[2], rb;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch = [&](int slab) {
+        const int k0 = slab * BK;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int e = tid + q * 256;
-            int kk, mm;
-            if (TA) { mm = e % BM; kk = e / BM; } else { kk = e % BK; mm = e / BK; }
-            const int gm = m0 + mm, gk = k0 + kk;
-            ra[q] = (gm < M && gk < kend) ? (TA ? A[(int64_t)gk * lda + gm] : A[(int64_t)gm * lda + gk]) : 0.f;
-            int kb, nn;
-            if (TB) { kb = e % BK; nn = e / BK; } else { nn = e % BN; kb = e / BN; }
-            const int gn = n0 + nn, gkb = k0 + kb;
-            rb[q] = (gn < N && gkb < kend) ? (TB ? B[(int64_t)gn * ldb + gkb] : B[(int64_t)gkb * ldb + gn]) : 0.f;
+        for (int q = 0; q < 2; q++) {
+            const int gm = m0 + row + 64 * q;
+            ra[q] = gm < M ? load4<VEC>(A + (int64_t)gm * H + k0 + kq) : zero;
+        }
+        if (TB) {
+            rb = load4<VEC>(W + (int64_t)(n0 + row) * H + k0 + kq);
+        } else {
+            copy4<VEC>(&Bs[slab % STAGES][tid / 16][tx * 4], W + (int64_t)(k0 + tid / 16) * H + n0 + tx * 4, true);
+            copies_end();
         }
     };
-    auto sstore = [&](int buf) {
+    auto settle = [&](int slab) {
+        const int st = slab % STAGES;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int e = tid + q * 256;
-            int kk, mm;
-            if (TA) { mm = e % BM; kk = e / BM; } else { kk = e % BK; mm = e / BK; }
-            As[buf][kk][mm] = ra[q];
-            int kb, nn;
-            if (TB) { kb = e % BK; nn = e / BK; } else { nn = e % BN; kb = e / BN; }
-            Bs[buf][kb][nn] = rb[q];
+        for (int q = 0; q < 2; q++) {
+            As[st][kq][row + 64 * q] = ra[q].x;
+            As[st][kq + 1][row + 64 * q] = ra[q].y;
+            As[st][kq + 2][row + 64 * q] = ra[q].z;
+            As[st][kq + 3][row + 64 * q] = ra[q].w;
+        }
+        if (TB) {
+            Bs[st][kq][row] = rb.x;
+            Bs[st][kq + 1][row] = rb.y;
+            Bs[st][kq + 2][row] = rb.z;
+            Bs[st][kq + 3][row] = rb.w;
         }
     };
-    gload(kbeg);
-    sstore(0);
+    uint64_t acc[4][4] = {};
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        fetch(s);
+        settle(s);
+    }
+    for (int s = 0; s < SLABS; s++) {
+        if (!TB) copies_wait<1>();
+        __syncthreads();
+        if (s + 2 < SLABS) fetch(s + 2);
+        else if (!TB) copies_end();
+        slab_product(acc, As[s % STAGES], Bs[s % STAGES], tx, ty);
+        if (s + 2 < SLABS) settle(s + 2);
+    }
+    const int gn = n0 + tx * 4;
+    const float4 bias = EPI == EPI_ACT || EPI == EPI_LAST ? load4<VEC>(ep.bias + gn) : zero;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        // both rows' operands are read before either is stored: the compiler may not do so
+        float4 s[2], t[2], u[2];
+        float e[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int gm = m0 + tile_row(i, r, ty);
+            if (gm >= M) continue;
+            const int64_t o = (int64_t)gm * H + gn;
+            if (EPI != EPI_ACT) s[r] = load4<VEC>(ep.S + o);
+            if (EPI == EPI_ADJ || EPI == EPI_LAST) t[r] = load4<VEC>(ep.T + o);
+            if (EPI == EPI_ADJ) u[r] = load4<VEC>(ep.U + o);
+            if (EPI == EPI_MAC) u[r] = load4<VEC>(C + o);
+            if (EPI == EPI_LAST) e[r] = ep.e[gm];
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int gm = m0 + tile_row(i, r, ty);
+            if (gm >= M) continue;
+            const int64_t o = (int64_t)gm * H + gn;
+            const float4 d = tile_values(acc[i], r);
+            if (EPI == EPI_ACT) {
+                float4 a, p, q;
+                silu3(d.x + bias.x, a.x, p.x, q.x);
+                silu3(d.y + bias.y, a.y, p.y, q.y);
+                silu3(d.z + bias.z, a.z, p.z, q.z);
+                silu3(d.w + bias.w, a.w, p.w, q.w);
+                store4<VEC>(C + o, a);
+                store4<VEC>(ep.p + o, p);
+                store4<VEC>(ep.q + o, q);
+            } else if (EPI == EPI_UD) {
+                store4<VEC>(C + o, d);
+                store4<VEC>(ep.p + o, d * s[r]);
+            } else if (EPI == EPI_ADJ) {
+                store4<VEC>(C + o, d * s[r]);
+                store4<VEC>(ep.p + o, d * u[r] * t[r]);
+            } else if (EPI == EPI_LAST) {
+                store4<VEC>(C + o, d * s[r]);
+                store4<VEC>(ep.p + o, make_float4(bias.x * (d.x * t[r].x + e[r] * s[r].x), bias.y * (d.y * t[r].y + e[r] * s[r].y),
+                                                  bias.z * (d.z * t[r].z + e[r] * s[r].z), bias.w * (d.w * t[r].w + e[r] * s[r].w)));
+            } else {
+                store4<VEC>(C + o, make_float4(u[r].x + d.x * s[r].x, u[r].y + d.y * s[r].y, u[r].z + d.z * s[r].z,
+                                               u[r].w + d.w * s[r].w));
+            }
+        }
+    }
+}
+
+// C[H,H] += sum over the rows b of the batch of A[b,:]^T B[b,:], each CTA of a tile over
+// its share of the batch (gridDim.z shares, so that the 8 tiles fill two CTAs on every
+// SM), four columns to an addition.
+// 256 x 256 x 8,192: 56 -> 25 us.
+template <bool VEC>
+__global__ void __launch_bounds__(256, 2) grads_kernel(int64_t batch, int share, const float *__restrict__ A,
+                                                       const float *__restrict__ B, float *__restrict__ C) {
+    __shared__ __align__(16) SlabA As[STAGES];
+    __shared__ __align__(16) SlabB Bs[STAGES];
+    const int tid = threadIdx.x;
+    const int tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int64_t kbeg = (int64_t)blockIdx.z * share;
+    const int64_t kend = min(batch, kbeg + share);
+    if (kbeg >= kend) return;
+    const int slabs = (int)((kend - kbeg + BK - 1) / BK);
+    auto fetch = [&](int slab) {
+        const int64_t k0 = kbeg + (int64_t)slab * BK;
+        const int st = slab % STAGES;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int e = tid + 256 * q, kk = e / 32, mm = e % 32 * 4;
+            const bool in = k0 + kk < kend;
+            copy4<VEC>(&As[st][kk][mm], A + (in ? k0 + kk : 0) * H + m0 + mm, in);
+        }
+        const bool in = k0 + ty < kend;
+        copy4<VEC>(&Bs[st][ty][tx * 4], B + (in ? k0 + ty : 0) * H + n0 + tx * 4, in);
+        copies_end();
+    };
+    uint64_t acc[4][4] = {};
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        if (s < slabs) fetch(s);
+        else copies_end();
+    }
+    for (int s = 0; s < slabs; s++) {
+        copies_wait<1>();
+        __syncthreads();
+        if (s + 2 < slabs) fetch(s + 2);
+        else copies_end();
+        slab_product(acc, As[s % STAGES], Bs[s % STAGES], tx, ty);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float *c = C + (int64_t)(m0 + tile_row(i, r, ty)) * H + n0 + tx * 4;
+            const float4 d = tile_values(acc[i], r);
+            if (VEC) {
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(c), "f"(d.x), "f"(d.y), "f"(d.z),
+                             "f"(d.w)
+                             : "memory");
+            } else {
+                atomicAdd(c, d.x);
+                atomicAdd(c + 1, d.y);
+                atomicAdd(c + 2, d.z);
+                atomicAdd(c + 3, d.w);
+            }
+        }
+    }
+}
+
+template <typename... P>
+static bool aligned16(const P *...p) {
+    return ((... | reinterpret_cast<uintptr_t>(p)) & 15) == 0;
+}
+
+// C = A op(W) with its epilogue
+template <bool TB, int EPI>
+static void rows(cudaStream_t st, int64_t batch, const float *A, const float *W, float *C, const Epi &ep) {
+    const dim3 grid(H / BN, nblk(batch, BM));
+    if (aligned16(A, W, C, ep.bias, ep.S, ep.U, ep.T, ep.p, ep.q))
+        rows_kernel<TB, EPI, true><<<grid, 256, 0, st>>>((int)batch, A, W, C, ep);
+    else
+        rows_kernel<TB, EPI, false><<<grid, 256, 0, st>>>((int)batch, A, W, C, ep);
+}
+
+// C += A^T B over the batch
+static void weight_grads(cudaStream_t st, int64_t batch, const float *A, const float *B, float *C) {
+    constexpr int TILES = (H / BM) * (H / BN);
+    const int64_t split = 2 * 152 / TILES;
+    const int share = (int)(((batch + split - 1) / split + BK - 1) / BK * BK);
+    const dim3 grid(H / BN, H / BM, nblk(batch, share));
+    if (aligned16(A, B, C))
+        grads_kernel<true><<<grid, 256, 0, st>>>(batch, share, A, B, C);
+    else
+        grads_kernel<false><<<grid, 256, 0, st>>>(batch, share, A, B, C);
+}
+
+// G[b, 0..2] = D[b, :] W with W [H][3] (one warp per row; as a 128-wide tile 38 us, now 7)
+__global__ void rows3_kernel(int64_t B, const float *__restrict__ D, const float *__restrict__ W, float *__restrict__ G) {
+    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (row >= B) return;
+    float g0 = 0.f, g1 = 0.f, g2 = 0.f;
+    for (int k = lane; k < H; k += 32) {
+        const float d = D[row * H + k];
+        g0 = fmaf(d, W[3 * k], g0);
+        g1 = fmaf(d, W[3 * k + 1], g1);
+        g2 = fmaf(d, W[3 * k + 2], g2);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        g0 += __shfl_xor_sync(0xffffffffu, g0, o);
+        g1 += __shfl_xor_sync(0xffffffffu, g1, o);
+        g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+    }
+    if (lane < 3) G[row * 3 + lane] = lane == 0 ? g0 : lane == 1 ? g1 : g2;
+}
+
+// Rows of the batch per CTA of the column reductions: 8,192 rows are 256 CTAs (as 32
+// CTAs of 256 rows a column sum took 21 us, now 6).
+constexpr int COL_ROWS = 32;
+
+// W[k, 0..2] += sum_b X[b, k] Y[b, 0..2], and with `sum` sum[k] += sum_b X[b, k] (as
+// 128-wide tiles 51 us, now 12)
+__global__ void cols3_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ Y, float *__restrict__ W,
+                             float *__restrict__ sum) {
+    const int k = threadIdx.x;  // blockDim = H
+    const int64_t r0 = (int64_t)blockIdx.x * COL_ROWS;
+    const int rows = (int)min((int64_t)COL_ROWS, B - r0);
+    __shared__ float y[3 * COL_ROWS];
+    if (k < 3 * rows) y[k] = Y[3 * r0 + k];
     __syncthreads();
-    int buf = 0;
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        const bool more = k0 + BK < kend;
-        if (more) gload(k0 + BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float a[8], b[8];
-            const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][64 + tx * 4]);
-            a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
-            b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w; b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        if (more) {
-            sstore(buf ^ 1);
-            __syncthreads();
-            buf ^= 1;
-        }
+    float w0 = 0.f, w1 = 0.f, w2 = 0.f, s = 0.f;
+#pragma unroll 16
+    for (int r = 0; r < COL_ROWS; r++) {
+        const float x = r < rows ? X[(r0 + r) * H + k] : 0.f;
+        w0 = fmaf(x, r < rows ? y[3 * r] : 0.f, w0);
+        w1 = fmaf(x, r < rows ? y[3 * r + 1] : 0.f, w1);
+        w2 = fmaf(x, r < rows ? y[3 * r + 2] : 0.f, w2);
+        s += x;
     }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-            if (gn >= N) continue;
-            float *c = &C[(int64_t)gm * ldc + gn];
-            if (gridDim.z > 1)
-                atomicAdd(c, alpha * acc[i][j]);  // split-K: C already holds beta * C
-            else
-                *c = alpha * acc[i][j] + (beta == 0.f ? 0.f : beta * *c);
-        }
-    }
+    atomicAdd(&W[3 * k], w0);
+    atomicAdd(&W[3 * k + 1], w1);
+    atomicAdd(&W[3 * k + 2], w2);
+    if (sum) atomicAdd(&sum[k], s);
 }
 
-// Split K over extra CTAs when the output tile grid is small (weight gradients:
-// 256 x 256 outputs, K = batch).  Split-K accumulates into C, so it is used
-// only with beta = 1.
-template <bool TA, bool TB>
-static void gemm(cudaStream_t st, int M, int N, int K, float alpha, const float *A, int lda, const float *B,
-                 int ldb, float beta, float *C, int ldc) {
-    const int tiles = ((N + 127) / 128) * ((M + 127) / 128);
-    int split = 1;
-    if (beta == 1.f && tiles < 152) {
-        split = (2 * 152 + tiles - 1) / tiles;
-        const int maxsplit = (K + 255) / 256;
-        if (split > maxsplit) split = maxsplit;
-        if (split < 1) split = 1;
-    }
-    dim3 grid((N + 127) / 128, (M + 127) / 128, split);
-    gemm_f32<TA, TB><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-}
-
-// Z (already A W^T, in place in `a`) + bias -> a = silu, s = silu', t = silu''.
-__global__ void act_kernel(int64_t n, const float *__restrict__ bias, float *__restrict__ a, float *__restrict__ s,
-                           float *__restrict__ t) {
+// The adjoint of G = D_1 W_1 for the first layer: d = E W_1^T, Ubar = d * S, Zbar = d * U * T
+__global__ void adj1_kernel(int64_t n, const float *__restrict__ E, const float *__restrict__ W1, const float *__restrict__ S,
+                            const float *__restrict__ U, const float *__restrict__ T, float *__restrict__ Ubar,
+                            float *__restrict__ Zbar) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float z = a[i] + bias[i % H];
-    float av, s1, s2;
-    silu3(z, av, s1, s2);
-    a[i] = av;
-    s[i] = s1;
-    t[i] = s2;
+    const int64_t b = i / H;
+    const int k = (int)(i % H);
+    const float d = fmaf(E[b * 3 + 2], W1[3 * k + 2], fmaf(E[b * 3 + 1], W1[3 * k + 1], E[b * 3] * W1[3 * k]));
+    Ubar[i] = d * S[i];
+    Zbar[i] = d * U[i] * T[i];
 }
 
 // out[b] = dot(A[b,:], w) + c  (one warp per row)
@@ -161,13 +405,6 @@ __global__ void d4_kernel(int64_t n, const float *__restrict__ w5, const float *
                           float *__restrict__ D4) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) D4[i] = w5[i % H] * S4[i];
-}
-
-// out = x * y (elementwise)
-__global__ void mul_kernel(int64_t n, const float *__restrict__ x, const float *__restrict__ y,
-                           float *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = x[i] * y[i];
 }
 
 // loss terms and their seeds: e = 2 alpha (y - y*) / B, E = 2 beta w (G - G*) / B
@@ -200,43 +437,18 @@ __global__ void loss_kernel(int64_t B, float alpha, float beta, const float *__r
     }
 }
 
-// Ubar = Dbar * S ; Zbar = Dbar * U * T
-__global__ void adj_kernel(int64_t n, const float *__restrict__ Dbar, const float *__restrict__ S,
-                           const float *__restrict__ U, const float *__restrict__ T, float *__restrict__ Ubar,
-                           float *__restrict__ Zbar) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float d = Dbar[i];
-    Ubar[i] = d * S[i];
-    Zbar[i] = d * U[i] * T[i];
-}
-
-// Zbar4 = Dbar4 * w5 * T4 + e * w5 * S4
-__global__ void zbar4_kernel(int64_t n, const float *__restrict__ Dbar4, const float *__restrict__ w5,
-                             const float *__restrict__ T4, const float *__restrict__ S4, const float *__restrict__ e,
-                             float *__restrict__ Zbar4) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int k = (int)(i % H);
-    Zbar4[i] = w5[k] * (Dbar4[i] * T4[i] + e[i / H] * S4[i]);
-}
-
-// Zbar += Abar * S
-__global__ void addmul_kernel(int64_t n, const float *__restrict__ Abar, const float *__restrict__ S,
-                              float *__restrict__ Zbar) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) Zbar[i] += Abar[i] * S[i];
-}
-
 // column sums over the batch: out[k] = sum_b X[b, k] (+ sum_b e[b] Y[b, k] if e)
 __global__ void colsum_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ e,
                               const float *__restrict__ Y, float *__restrict__ out) {
     const int k = threadIdx.x;  // blockDim = H
-    const int64_t r0 = (int64_t)blockIdx.x * 256;
+    const int64_t r0 = (int64_t)blockIdx.x * COL_ROWS;
+    const int rows = (int)min((int64_t)COL_ROWS, B - r0);
     float acc = 0.f;
-    for (int64_t r = r0; r < r0 + 256 && r < B; r++) {
-        acc += X[r * H + k];
-        if (e) acc += e[r] * Y[r * H + k];
+#pragma unroll 16
+    for (int r = 0; r < COL_ROWS; r++) {
+        const bool in = r < rows;
+        acc += in ? X[(r0 + r) * H + k] : 0.f;
+        if (e) acc += in ? e[r0 + r] * Y[(r0 + r) * H + k] : 0.f;
     }
     atomicAdd(&out[k], acc);
 }
@@ -280,7 +492,6 @@ __global__ void adam_kernel(int64_t n, float *__restrict__ p, const float *__res
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 }  // namespace mlp
 }  // namespace gx
@@ -307,17 +518,22 @@ extern "C" int gx_mlp_forward(const float *params, const float *xh, int64_t B, f
     for (int l = 1; l <= 3; l++) { U[l] = w; w += n; }
     layer1_kernel<<<nblk(n, 256), 256, 0, st>>>(B, xh, params, A[1], S[1], T[1]);
     for (int l = 2; l <= 4; l++) {
-        gemm<false, true>(st, (int)B, H, H, 1.f, A[l - 1], H, params + off_W(l), H, 0.f, A[l], H);
-        act_kernel<<<nblk(n, 256), 256, 0, st>>>(n, params + off_b(l), A[l], S[l], T[l]);
+        Epi ep = {};
+        ep.bias = params + off_b(l);
+        ep.p = S[l];
+        ep.q = T[l];
+        rows<true, EPI_ACT>(st, B, A[l - 1], params + off_W(l), A[l], ep);
     }
     rowdot_kernel<<<nblk(B * 32, 256), 256, 0, st>>>(B, A[4], params + OFF_W5, params + OFF_B5, y);
     if (G) {
         d4_kernel<<<nblk(n, 256), 256, 0, st>>>(n, params + OFF_W5, S[4], D[4]);
         for (int l = 3; l >= 1; l--) {
-            gemm<false, false>(st, (int)B, H, H, 1.f, D[l + 1], H, params + off_W(l + 1), H, 0.f, U[l], H);
-            mul_kernel<<<nblk(n, 256), 256, 0, st>>>(n, U[l], S[l], D[l]);
+            Epi ep = {};
+            ep.S = S[l];
+            ep.p = D[l];
+            rows<false, EPI_UD>(st, B, D[l + 1], params + off_W(l + 1), U[l], ep);
         }
-        gemm<false, false>(st, (int)B, 3, H, 1.f, D[1], H, params + OFF_W1, 3, 0.f, G, 3);
+        rows3_kernel<<<nblk(B * 32, 256), 256, 0, st>>>(B, D[1], params + OFF_W1, G);
     }
     return gx::check_launch("mlp_forward");
 }
@@ -340,7 +556,7 @@ extern "C" int gx_mlp_train_step(const float *params, float *grads, const float 
     for (int l = 1; l <= 3; l++) { U[l] = w; w += n; }
     float *Zb[5];
     for (int l = 1; l <= 4; l++) { Zb[l] = w; w += n; }
-    float *Dbar = w; w += n;
+    w += n;
     float *Ubar = w; w += n;
     float *Abar = w; w += n;
     float *y = w; w += B;
@@ -358,31 +574,43 @@ extern "C" int gx_mlp_train_step(const float *params, float *grads, const float 
     loss_kernel<<<nblk(B, 256), 256, 0, st>>>(B, alpha, beta, y, ystar, G, Gstar, gweight, e, E, loss);
 
     // adjoint of the input-gradient pass
-    gemm<true, false>(st, H, 3, (int)B, 1.f, D[1], H, E, 3, 1.f, g + OFF_W1, 3);      // W1g += D1^T E
-    // Dbar_1 = E W1^T : [B,3] x [3,256] where W1 is [256][3] -> B operand stored [N][K]
-    gemm<false, true>(st, (int)B, H, 3, 1.f, E, 3, params + OFF_W1, 3, 0.f, Dbar, H);
+    const unsigned cols = nblk(B, COL_ROWS);
+    cols3_kernel<<<cols, H, 0, st>>>(B, D[1], E, g + OFF_W1, nullptr);  // W1g += D1^T E
+    adj1_kernel<<<nblk(n, 256), 256, 0, st>>>(n, E, params + OFF_W1, S[1], U[1], T[1], Ubar, Zb[1]);
     for (int l = 1; l <= 3; l++) {
-        adj_kernel<<<nblk(n, 256), 256, 0, st>>>(n, Dbar, S[l], U[l], T[l], Ubar, Zb[l]);
         // W_{l+1} g += D_{l+1}^T Ubar_l  : [256 x B] x [B x 256]
-        gemm<true, false>(st, H, H, (int)B, 1.f, D[l + 1], H, Ubar, H, 1.f, g + off_W(l + 1), H);
-        // Dbar_{l+1} = Ubar_l W_{l+1}^T
-        gemm<false, true>(st, (int)B, H, H, 1.f, Ubar, H, params + off_W(l + 1), H, 0.f, Dbar, H);
+        weight_grads(st, B, D[l + 1], Ubar, g + off_W(l + 1));
+        // Dbar_{l+1} = Ubar_l W_{l+1}^T, and what follows it
+        Epi ep = {};
+        ep.S = S[l + 1];
+        ep.T = T[l + 1];
+        ep.p = Zb[l + 1];
+        if (l < 3) {
+            ep.U = U[l + 1];
+            rows<true, EPI_ADJ>(st, B, Ubar, params + off_W(l + 1), Abar, ep);
+            float *next = Ubar;
+            Ubar = Abar;
+            Abar = next;
+        } else {
+            // Abar = Dbar4 * S4 ; Zbar4 = w5 * (Dbar4 * T4 + e * S4)
+            ep.bias = W5;
+            ep.e = e;
+            rows<true, EPI_LAST>(st, B, Ubar, params + off_W(4), Abar, ep);
+        }
     }
-    // w5g += colsum(Dbar4 * S4) + A4^T e ; Zbar4 = w5 * (Dbar4 * T4 + e * S4)
-    mul_kernel<<<nblk(n, 256), 256, 0, st>>>(n, Dbar, S[4], Abar);
-    colsum_kernel<<<nblk(B, 256), H, 0, st>>>(B, Abar, e, A[4], g + OFF_W5);
-    zbar4_kernel<<<nblk(n, 256), 256, 0, st>>>(n, Dbar, W5, T[4], S[4], e, Zb[4]);
+    // w5g += colsum(Dbar4 * S4) + A4^T e
+    colsum_kernel<<<cols, H, 0, st>>>(B, Abar, e, A[4], g + OFF_W5);
     // b5g = sum e
     sum_kernel<<<nblk(B, 256), 256, 0, st>>>(B, e, g + OFF_B5);
     // backprop through the forward pass
     for (int l = 4; l >= 2; l--) {
-        gemm<true, false>(st, H, H, (int)B, 1.f, Zb[l], H, A[l - 1], H, 1.f, g + off_W(l), H);  // W_l g += Zbar^T A
-        colsum_kernel<<<nblk(B, 256), H, 0, st>>>(B, Zb[l], nullptr, nullptr, g + off_b(l));
-        gemm<false, false>(st, (int)B, H, H, 1.f, Zb[l], H, params + off_W(l), H, 0.f, Abar, H);  // Abar = Zbar W_l
-        addmul_kernel<<<nblk(n, 256), 256, 0, st>>>(n, Abar, S[l - 1], Zb[l - 1]);
+        weight_grads(st, B, Zb[l], A[l - 1], g + off_W(l));  // W_l g += Zbar^T A
+        colsum_kernel<<<cols, H, 0, st>>>(B, Zb[l], nullptr, nullptr, g + off_b(l));
+        Epi ep = {};
+        ep.S = S[l - 1];
+        rows<false, EPI_MAC>(st, B, Zb[l], params + off_W(l), Zb[l - 1], ep);  // Zbar_{l-1} += (Zbar_l W_l) * S
     }
-    gemm<true, false>(st, H, 3, (int)B, 1.f, Zb[1], H, xh, 3, 1.f, g + OFF_W1, 3);  // W1g += Zbar1^T X
-    colsum_kernel<<<nblk(B, 256), H, 0, st>>>(B, Zb[1], nullptr, nullptr, g + OFF_B1);
+    cols3_kernel<<<cols, H, 0, st>>>(B, Zb[1], xh, g + OFF_W1, g + OFF_B1);  // W1g += Zbar1^T X, b1g
     return gx::check_launch("mlp_train_step");
 }
 
