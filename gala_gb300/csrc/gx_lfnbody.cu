@@ -44,6 +44,9 @@ struct LfArgs {
     double *stream_w_out, *nbody_w_out;
     int32_t *status;
     int32_t gs;             // lanes per group (the largest system)
+    // release systems larger than max_per_release said go in a launch of their own:
+    int32_t upto;           // systems of more members than this get status -1
+    int32_t over;           // > 0: only systems of more members than this are this launch's
 };
 
 // Gradient at the lane's body, x after this step's drift and xo before it.  All 32
@@ -87,17 +90,18 @@ __global__ void __launch_bounds__(32) lf_nbody_kernel(const __grid_constant__ De
             si = sys / A.n_streams;
             ss = sys - si * A.n_streams;
             const int64_t o0 = A.offset[si], o1 = A.offset[si + 1];
-            const bool bad = o1 < o0 || o0 < 0 || o1 > A.n_particles || A.nbody + (o1 - o0) > gs;
+            const int64_t size = A.nbody + (o1 - o0);
+            const bool rows = o1 >= o0 && o0 >= 0 && o1 <= A.n_particles;
+            const bool bad = !A.over && (!rows || size > A.upto);
+            const bool here = rows && o1 > o0 && size > A.over && size <= gs;
             if (member == 0) {
-                done = A.status + ss * A.n_release + si;
+                int32_t *const status = A.status + ss * A.n_release + si;
                 if (bad) (void)GX_DBG_CHECK(!bad, DBG_OFFSET, si, A.n_release);
-                if (bad || o1 == o0) {
-                    *done = bad ? -1 : 0;
-                    done = nullptr;
-                }
+                if (bad || (!A.over && o1 == o0)) *status = bad ? -1 : 0;
+                if (here) done = status;
             }
             bod = A.bodies + ss * A.nbody;
-            in_sys = !bad && o1 > o0 && member < A.nbody + (int)(o1 - o0);
+            in_sys = here && member < (int)size;
             if (in_sys) {
                 n_steps = (int64_t)((A.t_final - A.release_t[si]) / dt + 0.5);  // mockstream.pyx:582
                 if (member < A.nbody) {
@@ -119,6 +123,7 @@ __global__ void __launch_bounds__(32) lf_nbody_kernel(const __grid_constant__ De
             }
         }
     }
+    if (STREAM && A.over && !__any_sync(0xffffffffu, in_sys)) return;
     int64_t most = n_steps;  // the warp's longest system
     for (int k = 16; k > 0; k >>= 1) {
         const int64_t other = __shfl_xor_sync(0xffffffffu, most, k);
@@ -164,13 +169,20 @@ int launch_lf(const DevPot &dp, LfArgs A, int members, cudaStream_t st) {
         set_error("leapfrog n-body systems of %d bodies: at most 8", members);
         return GX_ERR_UNSUPPORTED;
     }
-    A.gs = members;
-    const int64_t per = 32 / members;
-    const unsigned grid = (unsigned)((A.n_sys + per - 1) / per);
-    if (dp.has_scf)
-        lf_nbody_kernel<STREAM, SAVE_ALL, true><<<grid, 32, 0, st>>>(dp, A);
-    else
-        lf_nbody_kernel<STREAM, SAVE_ALL, false><<<grid, 32, 0, st>>>(dp, A);
+    // max_per_release sizes the groups; releases beyond it, up to three or eight
+    // members, are taken all the same, by groups of that size
+    const int most = dp.has_scf || members > 3 ? 8 : 3;
+    A.upto = most;
+    for (A.gs = members;; A.gs = most) {
+        const int64_t per = 32 / A.gs;
+        const unsigned grid = (unsigned)((A.n_sys + per - 1) / per);
+        if (dp.has_scf)
+            lf_nbody_kernel<STREAM, SAVE_ALL, true><<<grid, 32, 0, st>>>(dp, A);
+        else
+            lf_nbody_kernel<STREAM, SAVE_ALL, false><<<grid, 32, 0, st>>>(dp, A);
+        if (!STREAM || A.gs == most) break;
+        A.over = members;
+    }
     return check_launch(STREAM ? "mockstream_leapfrog" : "nbody_leapfrog");
 }
 
