@@ -55,6 +55,8 @@ def call_staged(name, head, a, out_size):
     host[:size].reshape(a.shape)[...] = a
     p = block.data_ptr()
     s = torch.cuda.current_stream()
-    _abi.call(name, *head, p, a.shape[1], p + 8 * size, int(s.cuda_stream))
-    s.synchronize()
+    try:
+        _abi.call(name, *head, p, a.shape[1], p + 8 * size, int(s.cuda_stream))
+    finally:  # the block is not given back before the kernel is done with it
+        s.synchronize()
     return host[size:].copy()
