@@ -1,12 +1,15 @@
-// gx_dop853.cu -- FP64 DOP853 with gala's batch semantics, one CTA per batch.
+// gx_dop853.cu -- FP64 DOP853 with gala's batch semantics.
 //
 // gala integrates `nbatch` orbits (default 100) as ONE ODE system of size
 // n = 6 * nb: one shared step size, one RMS error norm over all 6 * nb
 // components, one accept/reject decision, one dense-output grid
 // (dop853.pyx:228-245 -> dop853_helper :90-193 -> dopcor, dopri/dop853.cpp:89-650).
-// Here a batch is a group of consecutive threads of a CTA -- two batches per CTA
-// when that fills the warps better (100 orbits alone leave 28 idle lanes), the
-// two stepping in lock-step -- and each thread owns one orbit's six components:
+// Static frames take dop853_static_kernel below (a batch is a cluster of one-warp
+// CTAs), few orbits gx_dop853_axis.cu.  In the general kernel (rotating frames, small
+// or very large batches) a batch is a group of consecutive threads of a CTA -- two
+// batches per CTA when that fills the warps better (100 orbits alone leave 28 idle
+// lanes), the two stepping in lock-step -- and each thread owns one orbit's six
+// components:
 //   * the twelve stages, FSAL evaluation and the three dense-output stages are
 //     evaluated per thread in registers with gala's expression order;
 //   * the error norms (err, err2) and the stiffness sums (stnum, stden) are

@@ -431,7 +431,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 k5[c] = fma(h, k4[c], y[c]);
             }
 
-            // error estimation (:416-444), sequential over the system
+            // error estimation (:416-444)
             double err, err2;
             {
                 double t1[6], t2[6];
