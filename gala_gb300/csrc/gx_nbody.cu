@@ -18,7 +18,8 @@
 // body with its own potential shifted to body j's position.
 //
 // GPU mapping: a system is a GROUP of `gs` consecutive lanes of a warp, one
-// lane per body (32 / gs groups per warp).
+// lane per body (32 / gs groups per warp); few systems of up to ten bodies have a warp
+// each, three lanes per body.
 //   * Stage algebra runs per lane on its six components, in gala's term order
 //     as fused multiply-add chains, with the external force and the step
 //     controller in the FP64-pipe-lean forms of gx_fast64.cuh (this unit is
@@ -33,8 +34,11 @@
 //     the trajectory does not use it.
 //   * Few systems go one to a warp on SMs of their own: an FP64 instruction costs a
 //     warp 64 cycles whatever its lanes do, and four warps of an SM share one unit.
-//   127 systems of 9 bodies x 300 Myr, every tenth time kept: 21.0 -> 11.5 ms with the
-//   last four points (31 ms before the force left the FP64 pipe).
+//   * With three lanes to a body (NC = 2, a coordinate and its velocity each) the stage
+//     algebra is a third as long, and the lanes take a pulling body each and exchange
+//     the pulls' coordinates: a step is about 900 FP64 instructions instead of 1,300.
+//   127 systems of 9 bodies x 300 Myr, every tenth time kept: 31 ms before the force left
+//   the FP64 pipe, 21.0 after, 11.9 with the three points before the last, 7.3 now.
 //   * Groups take systems from a global counter, longest first; a group that
 //     finishes takes the next system at once, so a warp never idles on its
 //     slowest system.  Every loop is bounded by nmax like gala's.
@@ -151,21 +155,67 @@ __device__ __noinline__ V6 group_rhs_call(const DevPot &pot, const DevFrame &fr,
     return k;
 }
 
-template <bool SCF>
+// The same for one coordinate of the lane's body (static frames): the three lanes of a
+// body gather its position and take the external force alike, share the bodies that
+// pull, one each, and exchange the pulls' coordinates in two turns.
+struct V2 {
+    double x, v;
+};
+__device__ __noinline__ V2 axis_rhs_call(const DevPot &pot, int member, int nmem, int nbody,
+                                         const gx_body *__restrict__ bod, V2 in) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int axis = (threadIdx.x & 31) - 3 * member;
+    V3 q;
+#pragma unroll
+    for (int k = 0; k < 3; k++) q.v[k] = __shfl_sync(ALL, in.x, 3 * member + k);
+    const V3 a = fast::accel_call_f<false>(pot, q);
+    V2 out;
+    out.x = in.v;
+    out.v = axis == 0 ? a.v[0] : axis == 1 ? a.v[1] : a.v[2];
+    for (int j0 = 0; j0 < nbody; j0 += 3) {
+        const int j = j0 + axis;
+        double d[3], f[3] = {0., 0., 0.};
+#pragma unroll
+        for (int k = 0; k < 3; k++) d[k] = q.v[k] - __shfl_sync(ALL, in.x, 3 * j + k);
+        if (j < nbody && member != j && member < nmem) {
+            const int type = __ldg(&bod[j].type);
+            if (type != GX_POT_NULL) body_pull(type, bod[j].params, d[0], d[1], d[2], f);
+        }
+        // a lane keeps its own coordinate, sends the next two and takes its own from them
+        const double own = axis == 0 ? f[0] : axis == 1 ? f[1] : f[2];
+        const double nxt = axis == 0 ? f[1] : axis == 1 ? f[2] : f[0];
+        const double prv = axis == 0 ? f[2] : axis == 1 ? f[0] : f[1];
+        const double p = __shfl_sync(ALL, nxt, 3 * member + (axis == 0 ? 2 : axis - 1));
+        const double n = __shfl_sync(ALL, prv, 3 * member + (axis == 2 ? 0 : axis + 1));
+        out.v += own;
+        out.v += p;
+        out.v += n;
+    }
+    return out;
+}
+
+template <bool SCF, int NC>
 __device__ __forceinline__ void group_rhs(const DevPot &pot, const DevFrame &fr, unsigned mask, int base, int member,
                                           int nmem, int nbody, const gx_body *__restrict__ bod, const double *yin,
                                           double *kout) {
-    V6 a;
+    if constexpr (NC == 2) {
+        const V2 r = axis_rhs_call(pot, member, nmem, nbody, bod, V2{yin[0], yin[1]});
+        kout[0] = r.x;
+        kout[1] = r.v;
+    } else {
+        V6 a;
 #pragma unroll
-    for (int c = 0; c < 6; c++) a.v[c] = yin[c];
-    const V6 r = group_rhs_call<SCF>(pot, fr, mask, base, member, nmem, nbody, bod, a);
+        for (int c = 0; c < 6; c++) a.v[c] = yin[c];
+        const V6 r = group_rhs_call<SCF>(pot, fr, mask, base, member, nmem, nbody, bod, a);
 #pragma unroll
-    for (int c = 0; c < 6; c++) kout[c] = r.v[c];
+        for (int c = 0; c < 6; c++) kout[c] = r.v[c];
+    }
 }
 
-// Sums of two per-component series over the whole system: each lane's six terms in
+// Sums of two per-component series over the whole system: each lane's terms in
 // order, then the members' sums in order (a butterfly where the group's lanes are a
 // power of two, the lanes without a member adding zero).
+template <int NC>
 __device__ __forceinline__ void chain_sum2(unsigned mask, int gs, int span, int base, bool in_sys, const double *ta,
                                            const double *tb, double &sa, double &sb) {
     double a = 0.0, b = 0.0;
@@ -173,7 +223,7 @@ __device__ __forceinline__ void chain_sum2(unsigned mask, int gs, int span, int 
         a = ta[0];
         b = tb[0];
 #pragma unroll
-        for (int c = 1; c < 6; c++) {
+        for (int c = 1; c < NC; c++) {
             a += ta[c];
             b += tb[c];
         }
@@ -195,9 +245,9 @@ __device__ __forceinline__ void chain_sum2(unsigned mask, int gs, int span, int 
     }
 }
 
-#define GRHS(mask_, yin_, kout_) group_rhs<SCF>(pot, fr, (mask_), base, member, nmem, A.nbody, bod, (yin_), (kout_))
+#define GRHS(mask_, yin_, kout_) group_rhs<SCF, NC>(pot, fr, (mask_), base, member, nmem, A.nbody, bod, (yin_), (kout_))
 
-template <bool STREAM, bool DENSE, bool SCF>
+template <bool STREAM, bool DENSE, bool SCF, int NC>
 __global__ void __launch_bounds__(NB_THREADS)
 nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ DevFrame fr,
                     const __grid_constant__ NbArgs A) {
@@ -205,8 +255,12 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
     const int lane = threadIdx.x & 31;
     const int gs = A.gs, span = A.span;
     const int g = lane / span;
-    const int member = lane - g * span;
     const int base = g * span;
+    // six components to a lane, or (NC = 2, one system to the warp) a coordinate: x and v
+    const int member = NC == 6 ? lane - base : lane / 3;
+    const int axis = lane % 3;
+    const bool lead = lane == base;
+    const auto at = [&](int c) { return NC == 6 ? c : 3 * c + axis; };
     const bool lane_ok = g < 32 / span;
     const unsigned gmask = lane_ok ? (((span == 32) ? 0xffffffffu : ((1u << span) - 1u)) << base) : 0u;
 
@@ -214,7 +268,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
     const double facc1 = 1.0 / fac1, facc2 = 1.0 / fac2;
     const double atoli = A.atol, rtoli = A.rtol;
 
-    double y[6], k1[6], k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], k8[6], k9[6], k10[6], yy1[6];
+    double y[NC], k1[NC], k2[NC], k3[NC], k4[NC], k5[NC], k6[NC], k7[NC], k8[NC], k9[NC], k10[NC], yy1[NC];
     int64_t sys = 0, si = 0, ss = 0;
     int nmem = 0;
     const gx_body *bod = A.bodies;
@@ -227,9 +281,9 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
         // -- a group without a system takes the next one (group-local) --------
         if (!have && !done) {
             for (;;) {
-                // a cancelled launch takes no further system (member 0 decides for the group)
+                // a cancelled launch takes no further system (one lane decides for the group)
                 unsigned long long id = ~0ull;
-                if (member == 0 && !cancel_requested(A.cancel)) id = atomicAdd(A.counter, 1ull);
+                if (lead && !cancel_requested(A.cancel)) id = atomicAdd(A.counter, 1ull);
                 id = __shfl_sync(gmask, id, base);
                 if (id >= (unsigned long long)A.n_sys) {
                     done = true;
@@ -244,7 +298,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     // table inconsistent with the particle array (rejected, no access)
                     const bool bad = o1 < o0 || o0 < 0 || o1 > A.n_particles || o1 - o0 > gs - A.nbody;
                     if (o1 == o0 || bad) {
-                        if (member == 0) {
+                        if (lead) {
                             (void)GX_DBG_CHECK(!bad, DBG_OFFSET, si, A.n_release);
                             A.status[ss * A.n_release + si] = bad ? -1 : 0;
                             if (A.stats)
@@ -257,14 +311,14 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     if (member < A.nbody) {
                         const double *src = A.nbody_w + ((ss * A.n_release + si) * A.nbody + member) * 6;
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = src[c];
+                        for (int c = 0; c < NC; c++) y[c] = src[at(c)];
                     } else if (member < nmem) {
                         const double *src = A.stream_w0 + (ss * A.n_particles + o0 + (member - A.nbody)) * 6;
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = src[c];
+                        for (int c = 0; c < NC; c++) y[c] = src[at(c)];
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
+                        for (int c = 0; c < NC; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
                     }
                     // dop853_step's dop853() arguments (dop853.pyx:46-72) and front-end defaults
                     x = A.release_t[si];
@@ -279,10 +333,10 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     if (member < nmem) {
                         const double *src = A.w0 + (sys * A.nparticles + member) * 6;
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = src[c];
+                        for (int c = 0; c < NC; c++) y[c] = src[at(c)];
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 6; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
+                        for (int c = 0; c < NC; c++) y[c] = 1.;  // a lane without a member goes along at a harmless point
                     }
                     // dop853_helper's dop853() arguments (dop853.pyx:157-182)
                     x = A.t[0];
@@ -320,9 +374,9 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 GRHS(im, y, k1);
                 hmax = fabs(hmax);
                 if (h == 0.0) {
-                    double ta[6], tb[6];
+                    double ta[NC], tb[NC];
 #pragma unroll
-                    for (int c = 0; c < 6; c++) {
+                    for (int c = 0; c < NC; c++) {
                         const double sk = atoli + rtoli * fabs(y[c]);
                         double sqr = k1[c] / sk;
                         ta[c] = sqr * sqr;
@@ -330,22 +384,22 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                         tb[c] = sqr * sqr;
                     }
                     double dnf, dny;
-                    chain_sum2(im, gs, span, base, in_sys, ta, tb, dnf, dny);
+                    chain_sum2<NC>(im, gs, span, base, in_sys, ta, tb, dnf, dny);
                     double hh = ((dnf <= 1.0E-10) || (dny <= 1.0E-10)) ? 1.0E-6 : sqrt(dny / dnf) * 0.01;
                     hh = nb_min(hh, hmax);
                     hh = nb_sign(hh, posneg);
 #pragma unroll
-                    for (int c = 0; c < 6; c++) yy1[c] = y[c] + hh * k1[c];
+                    for (int c = 0; c < NC; c++) yy1[c] = y[c] + hh * k1[c];
                     GRHS(im, yy1, k2);
 #pragma unroll
-                    for (int c = 0; c < 6; c++) {
+                    for (int c = 0; c < NC; c++) {
                         const double sk = atoli + rtoli * fabs(y[c]);
                         const double sqr = (k2[c] - k1[c]) / sk;
                         ta[c] = sqr * sqr;
                         tb[c] = 0.;
                     }
                     double der2, unused;
-                    chain_sum2(im, gs, span, base, in_sys, ta, tb, der2, unused);
+                    chain_sum2<NC>(im, gs, span, base, in_sys, ta, tb, der2, unused);
                     der2 = sqrt(der2) / hh;
                     const double der12 = nb_max(fabs(der2), sqrt(dnf));
                     const double h1 =
@@ -380,52 +434,52 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
 
             // the twelve stages (dop853.cpp:368-414)
 #pragma unroll
-            for (int c = 0; c < 6; c++) yy1[c] = fma(h * a21, k1[c], y[c]);
+            for (int c = 0; c < NC; c++) yy1[c] = fma(h * a21, k1[c], y[c]);
             GRHS(am, yy1, k2);
 #pragma unroll
-            for (int c = 0; c < 6; c++) yy1[c] = fma(h, fma(a32, k2[c], a31 * k1[c]), y[c]);
+            for (int c = 0; c < NC; c++) yy1[c] = fma(h, fma(a32, k2[c], a31 * k1[c]), y[c]);
             GRHS(am, yy1, k3);
 #pragma unroll
-            for (int c = 0; c < 6; c++) yy1[c] = fma(h, fma(a43, k3[c], a41 * k1[c]), y[c]);
+            for (int c = 0; c < NC; c++) yy1[c] = fma(h, fma(a43, k3[c], a41 * k1[c]), y[c]);
             GRHS(am, yy1, k4);
 #pragma unroll
-            for (int c = 0; c < 6; c++) yy1[c] = fma(h, fma(a54, k4[c], fma(a53, k3[c], a51 * k1[c])), y[c]);
+            for (int c = 0; c < NC; c++) yy1[c] = fma(h, fma(a54, k4[c], fma(a53, k3[c], a51 * k1[c])), y[c]);
             GRHS(am, yy1, k5);
 #pragma unroll
-            for (int c = 0; c < 6; c++) yy1[c] = fma(h, fma(a65, k5[c], fma(a64, k4[c], a61 * k1[c])), y[c]);
+            for (int c = 0; c < NC; c++) yy1[c] = fma(h, fma(a65, k5[c], fma(a64, k4[c], a61 * k1[c])), y[c]);
             GRHS(am, yy1, k6);
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a76, k6[c], fma(a75, k5[c], fma(a74, k4[c], a71 * k1[c]))), y[c]);
             GRHS(am, yy1, k7);
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a87, k7[c], fma(a86, k6[c], fma(a85, k5[c], fma(a84, k4[c], a81 * k1[c])))), y[c]);
             GRHS(am, yy1, k8);
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a98, k8[c], fma(a97, k7[c], fma(a96, k6[c], fma(a95, k5[c],
                     fma(a94, k4[c], a91 * k1[c]))))), y[c]);
             GRHS(am, yy1, k9);
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a109, k9[c], fma(a108, k8[c], fma(a107, k7[c], fma(a106, k6[c], fma(a105, k5[c],
                     fma(a104, k4[c], a101 * k1[c])))))), y[c]);
             GRHS(am, yy1, k10);
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a1110, k10[c], fma(a119, k9[c], fma(a118, k8[c], fma(a117, k7[c], fma(a116, k6[c],
                     fma(a115, k5[c], fma(a114, k4[c], a111 * k1[c]))))))), y[c]);
             GRHS(am, yy1, k2);
             const double xph = x + h;
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+            for (int c = 0; c < NC; c++)
                 yy1[c] = fma(h, fma(a1211, k2[c], fma(a1210, k10[c], fma(a129, k9[c], fma(a128, k8[c], fma(a127, k7[c],
                     fma(a126, k6[c], fma(a125, k5[c], fma(a124, k4[c], a121 * k1[c])))))))), y[c]);
             GRHS(am, yy1, k3);
             nfcn += 11;
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
+            for (int c = 0; c < NC; c++) {
                 k4[c] = fma(b12, k3[c], fma(b11, k2[c], fma(b10, k10[c], fma(b9, k9[c], fma(b8, k8[c], fma(b7, k7[c],
                             fma(b6, k6[c], b1 * k1[c])))))));
                 k5[c] = fma(h, k4[c], y[c]);
@@ -434,9 +488,9 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
             // error estimation (:416-444)
             double err, err2;
             {
-                double t1[6], t2[6];
+                double t1[NC], t2[NC];
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
+                for (int c = 0; c < NC; c++) {
                     const double isk = fast::rcp_f(fma(rtoli, max_abs(y[c], k5[c]), atoli));
                     double erri = fma(-bhh3, k3[c], fma(-bhh2, k9[c], fma(-bhh1, k1[c], k4[c])));
                     double sqr = erri * isk;
@@ -446,7 +500,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     sqr = erri * isk;
                     t1[c] = sqr * sqr;
                 }
-                chain_sum2(am, gs, span, base, in_sys, t1, t2, err, err2);
+                chain_sum2<NC>(am, gs, span, base, in_sys, t1, t2, err, err2);
             }
             double deno = fma(0.01, err2, err);
             if (deno <= 0.0) deno = 1.0;
@@ -473,16 +527,16 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
             bool stiff = false;
             const bool test_st = acc && (!(naccpt % nstiff) || (iasti > 0));
             if (__ballot_sync(am, test_st)) {
-                double ta[6], tb[6];
+                double ta[NC], tb[NC];
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
+                for (int c = 0; c < NC; c++) {
                     double sqr = k4[c] - k3[c];
                     ta[c] = sqr * sqr;
                     sqr = k5[c] - yy1[c];
                     tb[c] = sqr * sqr;
                 }
                 double stnum, stden;
-                chain_sum2(am, gs, span, base, in_sys, ta, tb, stnum, stden);
+                chain_sum2<NC>(am, gs, span, base, in_sys, ta, tb, stnum, stden);
                 if (test_st) {
                     if (stden > 0.0) hlamb = h * dsqrt(ddiv(stnum, stden));
                     if (hlamb > 6.1) {
@@ -514,12 +568,12 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 }
                 // prepared by every group when one needs it, written by those that do
                 if (__ballot_sync(am, store)) {
-                    double r5[6], r6[6], r7[6], r8[6];
+                    double r5[NC], r6[NC], r7[NC], r8[NC];
 #define GX_D8(p)                                                                                                  \
     fma(p##12, k3[c], fma(p##11, k2[c], fma(p##10, k10[c], fma(p##9, k9[c], fma(p##8, k8[c], fma(p##7, k7[c],      \
         fma(p##6, k6[c], p##1 * k1[c])))))))
 #pragma unroll
-                    for (int c = 0; c < 6; c++) {
+                    for (int c = 0; c < NC; c++) {
                         r5[c] = fma(d413, k4[c], GX_D8(d4));
                         r6[c] = fma(d513, k4[c], GX_D8(d5));
                         r7[c] = fma(d613, k4[c], GX_D8(d6));
@@ -527,24 +581,24 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                     }
 #undef GX_D8
 #pragma unroll
-                    for (int c = 0; c < 6; c++)
+                    for (int c = 0; c < NC; c++)
                         yy1[c] = fma(h, fma(a1413, k4[c], fma(a1412, k3[c], fma(a1411, k2[c], fma(a1410, k10[c],
                             fma(a149, k9[c], fma(a148, k8[c], fma(a147, k7[c], a141 * k1[c]))))))), y[c]);
                     GRHS(am, yy1, k10);
 #pragma unroll
-                    for (int c = 0; c < 6; c++)
+                    for (int c = 0; c < NC; c++)
                         yy1[c] = fma(h, fma(a1514, k10[c], fma(a1513, k4[c], fma(a1512, k3[c], fma(a1511, k2[c],
                             fma(a158, k8[c], fma(a157, k7[c], fma(a156, k6[c], a151 * k1[c]))))))), y[c]);
                     GRHS(am, yy1, k2);
 #pragma unroll
-                    for (int c = 0; c < 6; c++)
+                    for (int c = 0; c < NC; c++)
                         yy1[c] = fma(h, fma(a1615, k2[c], fma(a1614, k10[c], fma(a1613, k4[c], fma(a169, k9[c],
                             fma(a168, k8[c], fma(a167, k7[c], fma(a166, k6[c], a161 * k1[c]))))))), y[c]);
                     GRHS(am, yy1, k3);
                     if (store) {
                         double *o = A.w_out + ((sys * A.n_out + out_slot) * A.nparticles + member) * 6;
 #pragma unroll
-                        for (int c = 0; c < 6; c++) {
+                        for (int c = 0; c < NC; c++) {
                             r5[c] = h * fma(d416, k3[c], fma(d415, k2[c], fma(d414, k10[c], r5[c])));
                             r6[c] = h * fma(d516, k3[c], fma(d515, k2[c], fma(d514, k10[c], r6[c])));
                             r7[c] = h * fma(d616, k3[c], fma(d615, k2[c], fma(d614, k10[c], r7[c])));
@@ -554,11 +608,11 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                             const double s = ddiv(A.t[kept] - xold, hout);
                             const double s1 = 1.0 - s;
 #pragma unroll
-                            for (int c = 0; c < 6; c++) {
+                            for (int c = 0; c < NC; c++) {
                                 const double ydiff = k5[c] - y[c], bspl = fma(h, k1[c], -ydiff);
                                 const double v = fma(s, fma(s1, fma(s, fma(s1, fma(s, fma(s1, fma(s, r8[c], r7[c]), r6[c]), r5[c]),
                                                                            fma(-h, k4[c], ydiff) - bspl), bspl), ydiff), y[c]);
-                                if (in_sys) o[c] = v;
+                                if (in_sys) o[at(c)] = v;
                             }
                         }
                     }
@@ -567,7 +621,7 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
 
             if (acc && !stiff) {
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
+                for (int c = 0; c < NC; c++) {
                     k1[c] = k4[c];
                     y[c] = k5[c];
                 }
@@ -595,15 +649,15 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 if (member >= A.nbody && member < nmem) {
                     double *o = A.stream_w_out + (ss * A.n_particles + o0 + (member - A.nbody)) * 6;
 #pragma unroll
-                    for (int c = 0; c < 6; c++) o[c] = y[c];
+                    for (int c = 0; c < NC; c++) o[at(c)] = y[c];
                 }
                 // the bodies after the last release system (mockstream.pyx:287-289)
                 if (member < A.nbody && A.nbody_w_out && A.offset[si + 1] == A.offset[A.n_release]) {
                     double *o = A.nbody_w_out + (ss * A.nbody + member) * 6;
 #pragma unroll
-                    for (int c = 0; c < 6; c++) o[c] = y[c];
+                    for (int c = 0; c < NC; c++) o[at(c)] = y[c];
                 }
-                if (member == 0) {
+                if (lead) {
                     const int64_t k = ss * A.n_release + si;
                     A.status[k] = idid;
                     if (A.stats) {
@@ -617,9 +671,9 @@ nbody_dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ 
                 if (!A.save_all && in_sys) {
                     double *o = A.w_out + (sys * A.nparticles + member) * 6;
 #pragma unroll
-                    for (int c = 0; c < 6; c++) o[c] = y[c];
+                    for (int c = 0; c < NC; c++) o[at(c)] = y[c];
                 }
-                if (member == 0) {
+                if (lead) {
                     A.status[sys] = idid;
                     if (A.stats) {
                         A.stats[4 * sys + 0] = nfcn;
@@ -793,12 +847,17 @@ int launch_nbody(const DevPot &dp, const DevFrame &df, NbArgs A, cudaStream_t st
     A.span = A.gs;
     for (int p = 1; p <= 32; p *= 2)
         if (p >= A.gs && (A.n_sys + 32 / p - 1) / (32 / p) <= 4 * (int64_t)sms) A.span = p;
-    if (dp.has_scf)
-        GX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nbody_dop853_kernel<STREAM, DENSE, true>,
-                                                                  NB_THREADS, 0));
-    else
-        GX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nbody_dop853_kernel<STREAM, DENSE, false>,
-                                                                  NB_THREADS, 0));
+    // Up to eight systems of at most ten bodies per SM, static frame: three lanes to a
+    // body, one system to a warp.  100 Myr around the MW composite, three lanes / one:
+    // 608 systems of 9 bodies 6.4 / 11.6 ms, 1,216 systems of 1, 3, 6, 10 bodies 4.8 /
+    // 6.1, 6.8 / 7.7, 7.1 / 9.4, 7.6 / 11.1 ms, 2,000 systems 5.6 / 6.7, 8.8 / 7.5,
+    // 10.4 / 9.8, 12.2 / 12.0 ms.
+    const bool axis = A.n_sys <= 8 * (int64_t)sms && A.gs <= 10 && df.type == GX_FRAME_STATIC && !dp.has_scf;
+    if (axis) A.span = 32;
+    const auto kernel = dp.has_scf ? nbody_dop853_kernel<STREAM, DENSE, true, 6>
+                        : axis     ? nbody_dop853_kernel<STREAM, DENSE, false, 2>
+                                   : nbody_dop853_kernel<STREAM, DENSE, false, 6>;
+    GX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NB_THREADS, 0));
     if (per_sm < 1) per_sm = 1;
     const int64_t groups_per_block = (int64_t)(NB_THREADS / 32) * (32 / A.span);
     int64_t need = (A.n_sys + groups_per_block - 1) / groups_per_block;
@@ -806,10 +865,7 @@ int launch_nbody(const DevPot &dp, const DevFrame &df, NbArgs A, cudaStream_t st
     if (need < grid) grid = need;
     if (grid < 1) grid = 1;
     GX_CUDA_TRY(cudaMemsetAsync(A.counter, 0, sizeof(unsigned long long), st));
-    if (dp.has_scf)
-        nbody_dop853_kernel<STREAM, DENSE, true><<<(unsigned)grid, NB_THREADS, 0, st>>>(dp, df, A);
-    else
-        nbody_dop853_kernel<STREAM, DENSE, false><<<(unsigned)grid, NB_THREADS, 0, st>>>(dp, df, A);
+    kernel<<<(unsigned)grid, NB_THREADS, 0, st>>>(dp, df, A);
     return check_launch(STREAM ? "mockstream_dop853" : "nbody_dop853");
 }
 
