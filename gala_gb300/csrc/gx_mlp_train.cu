@@ -18,9 +18,13 @@
 // Every 256-wide product is a tiled FP32 kernel (rows_kernel, with the elementwise pass
 // that follows it in its epilogue; grads_kernel for the weights); the products with the
 // 3-wide input or gradient are row and column reductions of their own.  What bounds a
-// step is the FP32 pipe: 18 products of batch x 256 x 256.  Batch 8,192, 16 steps: 21.1 -> 12.6 ms.
+// step is the FP32 pipe: 18 products of batch x 256 x 256.  Batch 8,192, 16 steps: 21.1 -> 12.5 ms.
+#include <cooperative_groups.h>
+
 #include "gx_host.h"
 #include "gx_mlp.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace gx {
 namespace mlp {
@@ -237,20 +241,28 @@ __global__ void __launch_bounds__(256, 2) rows_kernel(int M, const float *__rest
 
 // C[H,H] += sum over the rows b of the batch of A[b,:]^T B[b,:], each CTA of a tile over
 // its share of the batch (gridDim.z shares, so that the 8 tiles fill two CTAs on every
-// SM), four columns to an addition.
-// 256 x 256 x 8,192: 56 -> 25 us.
+// SM). Two CTAs of a cluster add their tiles before they add to C, four columns at a
+// time: half the additions in a row, whose rounding is most of the error (relative to
+// 64 bits, batch 4,096: 1.9e-7 alone, 1.5e-7 in pairs).
+// 256 x 256 x 8,192: 56 -> 26 us.
 template <bool VEC>
-__global__ void __launch_bounds__(256, 2) grads_kernel(int64_t batch, int share, const float *__restrict__ A,
+__global__ void __cluster_dims__(1, 1, 2) __launch_bounds__(256, 2) grads_kernel(int64_t batch, int share, const float *__restrict__ A,
                                                        const float *__restrict__ B, float *__restrict__ C) {
-    __shared__ __align__(16) SlabA As[STAGES];
-    __shared__ __align__(16) SlabB Bs[STAGES];
+    __shared__ __align__(16) union {
+        struct {
+            SlabA As[STAGES];
+            SlabB Bs[STAGES];
+        } in;
+        float4 tile[BM][BN / 4];
+    } sh;
+    SlabA *const As = sh.in.As;
+    SlabB *const Bs = sh.in.Bs;
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int64_t kbeg = (int64_t)blockIdx.z * share;
     const int64_t kend = min(batch, kbeg + share);
-    if (kbeg >= kend) return;
-    const int slabs = (int)((kend - kbeg + BK - 1) / BK);
+    const int slabs = kbeg < kend ? (int)((kend - kbeg + BK - 1) / BK) : 0;
     auto fetch = [&](int slab) {
         const int64_t k0 = kbeg + (int64_t)slab * BK;
         const int st = slab % STAGES;
@@ -277,24 +289,34 @@ __global__ void __launch_bounds__(256, 2) grads_kernel(int64_t batch, int share,
         else copies_end();
         slab_product(acc, As[s % STAGES], Bs[s % STAGES], tx, ty);
     }
+    copies_wait<0>();
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            float *c = C + (int64_t)(m0 + tile_row(i, r, ty)) * H + n0 + tx * 4;
-            const float4 d = tile_values(acc[i], r);
-            if (VEC) {
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(c), "f"(d.x), "f"(d.y), "f"(d.z),
-                             "f"(d.w)
-                             : "memory");
-            } else {
-                atomicAdd(c, d.x);
-                atomicAdd(c + 1, d.y);
-                atomicAdd(c + 2, d.z);
-                atomicAdd(c + 3, d.w);
-            }
+        for (int r = 0; r < 2; r++) sh.tile[tile_row(i, r, ty)][tx] = tile_values(acc[i], r);
+    // each CTA adds up half of the rows
+    cg::cluster_group pair = cg::this_cluster();
+    pair.sync();
+    const unsigned rank = pair.block_rank();
+    const float4(*const theirs)[BN / 4] = pair.map_shared_rank(sh.tile, rank ^ 1);
+#pragma unroll
+    for (int q = 0; q < BM / 2 / 16; q++) {
+        const int row = rank * (BM / 2) + 16 * q + ty;
+        const float4 a = sh.tile[row][tx], b = theirs[row][tx];
+        const float4 d = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+        float *c = C + (int64_t)(m0 + row) * H + n0 + tx * 4;
+        if (VEC) {
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(c), "f"(d.x), "f"(d.y), "f"(d.z), "f"(d.w)
+                         : "memory");
+        } else {
+            atomicAdd(c, d.x);
+            atomicAdd(c + 1, d.y);
+            atomicAdd(c + 2, d.z);
+            atomicAdd(c + 3, d.w);
         }
     }
+    pair.sync();  // the other CTA has read this one's tile
 }
 
 template <typename... P>
@@ -317,7 +339,7 @@ static void weight_grads(cudaStream_t st, int64_t batch, const float *A, const f
     constexpr int TILES = (H / BM) * (H / BN);
     const int64_t split = 2 * 152 / TILES;
     const int share = (int)(((batch + split - 1) / split + BK - 1) / BK * BK);
-    const dim3 grid(H / BN, H / BM, nblk(batch, share));
+    const dim3 grid(H / BN, H / BM, (nblk(batch, share) + 1) / 2 * 2);
     if (aligned16(A, B, C))
         grads_kernel<true><<<grid, 256, 0, st>>>(batch, share, A, B, C);
     else
@@ -345,33 +367,39 @@ __global__ void rows3_kernel(int64_t B, const float *__restrict__ D, const float
     if (lane < 3) G[row * 3 + lane] = lane == 0 ? g0 : lane == 1 ? g1 : g2;
 }
 
-// Rows of the batch per CTA of the column reductions: 8,192 rows are 256 CTAs (as 32
-// CTAs of 256 rows a column sum took 21 us, now 6).
-constexpr int COL_ROWS = 32;
+// The column reductions: a CTA takes 256 rows of the batch, four groups of 256 threads
+// 64 each, and adds the groups' sums before it adds to the result: 32 additions in a row
+// for 8,192 samples.  (With 256 rows to a thread a column sum took 21 us, now 8; with
+// 32 rows to a thread and 256 CTAs 6 us, but twice the rounding error.)
+constexpr int COL_GROUPS = 4, COL_ROWS = 64;
 
 // W[k, 0..2] += sum_b X[b, k] Y[b, 0..2], and with `sum` sum[k] += sum_b X[b, k] (as
-// 128-wide tiles 51 us, now 12)
-__global__ void cols3_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ Y, float *__restrict__ W,
-                             float *__restrict__ sum) {
-    const int k = threadIdx.x;  // blockDim = H
-    const int64_t r0 = (int64_t)blockIdx.x * COL_ROWS;
-    const int rows = (int)min((int64_t)COL_ROWS, B - r0);
-    __shared__ float y[3 * COL_ROWS];
-    if (k < 3 * rows) y[k] = Y[3 * r0 + k];
+// 128-wide tiles 51 us, now 9)
+__global__ void __launch_bounds__(COL_GROUPS *H) cols3_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ Y,
+                                                              float *__restrict__ W, float *__restrict__ sum) {
+    const int k = threadIdx.x % H, part = threadIdx.x / H;
+    const int64_t c0 = (int64_t)blockIdx.x * COL_GROUPS * COL_ROWS, r0 = c0 + part * COL_ROWS;
+    __shared__ float y[3 * COL_GROUPS * COL_ROWS], sums[COL_GROUPS][4][H];
+    if (threadIdx.x < 3 * COL_GROUPS * COL_ROWS) y[threadIdx.x] = 3 * c0 + threadIdx.x < 3 * B ? Y[3 * c0 + threadIdx.x] : 0.f;
     __syncthreads();
     float w0 = 0.f, w1 = 0.f, w2 = 0.f, s = 0.f;
 #pragma unroll 16
     for (int r = 0; r < COL_ROWS; r++) {
-        const float x = r < rows ? X[(r0 + r) * H + k] : 0.f;
-        w0 = fmaf(x, r < rows ? y[3 * r] : 0.f, w0);
-        w1 = fmaf(x, r < rows ? y[3 * r + 1] : 0.f, w1);
-        w2 = fmaf(x, r < rows ? y[3 * r + 2] : 0.f, w2);
+        const float x = r0 + r < B ? X[(r0 + r) * H + k] : 0.f;
+        const float *yr = y + 3 * (part * COL_ROWS + r);
+        w0 = fmaf(x, yr[0], w0);
+        w1 = fmaf(x, yr[1], w1);
+        w2 = fmaf(x, yr[2], w2);
         s += x;
     }
-    atomicAdd(&W[3 * k], w0);
-    atomicAdd(&W[3 * k + 1], w1);
-    atomicAdd(&W[3 * k + 2], w2);
-    if (sum) atomicAdd(&sum[k], s);
+    sums[part][0][k] = w0;
+    sums[part][1][k] = w1;
+    sums[part][2][k] = w2;
+    sums[part][3][k] = s;
+    __syncthreads();
+    const float total = (sums[0][part][k] + sums[1][part][k]) + (sums[2][part][k] + sums[3][part][k]);
+    if (part < 3) atomicAdd(&W[3 * k + part], total);
+    else if (sum) atomicAdd(&sum[k], total);
 }
 
 // The adjoint of G = D_1 W_1 for the first layer: d = E W_1^T, Ubar = d * S, Zbar = d * U * T
@@ -438,19 +466,21 @@ __global__ void loss_kernel(int64_t B, float alpha, float beta, const float *__r
 }
 
 // column sums over the batch: out[k] = sum_b X[b, k] (+ sum_b e[b] Y[b, k] if e)
-__global__ void colsum_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ e,
-                              const float *__restrict__ Y, float *__restrict__ out) {
-    const int k = threadIdx.x;  // blockDim = H
-    const int64_t r0 = (int64_t)blockIdx.x * COL_ROWS;
-    const int rows = (int)min((int64_t)COL_ROWS, B - r0);
+__global__ void __launch_bounds__(COL_GROUPS *H) colsum_kernel(int64_t B, const float *__restrict__ X, const float *__restrict__ e,
+                                                               const float *__restrict__ Y, float *__restrict__ out) {
+    const int k = threadIdx.x % H, part = threadIdx.x / H;
+    const int64_t r0 = ((int64_t)blockIdx.x * COL_GROUPS + part) * COL_ROWS;
+    __shared__ float sums[COL_GROUPS][H];
     float acc = 0.f;
 #pragma unroll 16
     for (int r = 0; r < COL_ROWS; r++) {
-        const bool in = r < rows;
+        const bool in = r0 + r < B;
         acc += in ? X[(r0 + r) * H + k] : 0.f;
         if (e) acc += in ? e[r0 + r] * Y[(r0 + r) * H + k] : 0.f;
     }
-    atomicAdd(&out[k], acc);
+    sums[part][k] = acc;
+    __syncthreads();
+    if (part == 0) atomicAdd(&out[k], (sums[0][k] + sums[1][k]) + (sums[2][k] + sums[3][k]));
 }
 
 // out += sum_b x[b]
@@ -574,8 +604,8 @@ extern "C" int gx_mlp_train_step(const float *params, float *grads, const float 
     loss_kernel<<<nblk(B, 256), 256, 0, st>>>(B, alpha, beta, y, ystar, G, Gstar, gweight, e, E, loss);
 
     // adjoint of the input-gradient pass
-    const unsigned cols = nblk(B, COL_ROWS);
-    cols3_kernel<<<cols, H, 0, st>>>(B, D[1], E, g + OFF_W1, nullptr);  // W1g += D1^T E
+    const unsigned cols = nblk(B, COL_GROUPS * COL_ROWS);
+    cols3_kernel<<<cols, COL_GROUPS * H, 0, st>>>(B, D[1], E, g + OFF_W1, nullptr);  // W1g += D1^T E
     adj1_kernel<<<nblk(n, 256), 256, 0, st>>>(n, E, params + OFF_W1, S[1], U[1], T[1], Ubar, Zb[1]);
     for (int l = 1; l <= 3; l++) {
         // W_{l+1} g += D_{l+1}^T Ubar_l  : [256 x B] x [B x 256]
@@ -599,18 +629,18 @@ extern "C" int gx_mlp_train_step(const float *params, float *grads, const float 
         }
     }
     // w5g += colsum(Dbar4 * S4) + A4^T e
-    colsum_kernel<<<cols, H, 0, st>>>(B, Abar, e, A[4], g + OFF_W5);
+    colsum_kernel<<<cols, COL_GROUPS * H, 0, st>>>(B, Abar, e, A[4], g + OFF_W5);
     // b5g = sum e
     sum_kernel<<<nblk(B, 256), 256, 0, st>>>(B, e, g + OFF_B5);
     // backprop through the forward pass
     for (int l = 4; l >= 2; l--) {
         weight_grads(st, B, Zb[l], A[l - 1], g + off_W(l));  // W_l g += Zbar^T A
-        colsum_kernel<<<cols, H, 0, st>>>(B, Zb[l], nullptr, nullptr, g + off_b(l));
+        colsum_kernel<<<cols, COL_GROUPS * H, 0, st>>>(B, Zb[l], nullptr, nullptr, g + off_b(l));
         Epi ep = {};
         ep.S = S[l - 1];
         rows<false, EPI_MAC>(st, B, Zb[l], params + off_W(l), Zb[l - 1], ep);  // Zbar_{l-1} += (Zbar_l W_l) * S
     }
-    cols3_kernel<<<cols, H, 0, st>>>(B, Zb[1], xh, g + OFF_W1, g + OFF_B1);  // W1g += Zbar1^T X, b1g
+    cols3_kernel<<<cols, COL_GROUPS * H, 0, st>>>(B, Zb[1], xh, g + OFF_W1, g + OFF_B1);  // W1g += Zbar1^T X, b1g
     return gx::check_launch("mlp_train_step");
 }
 
