@@ -469,9 +469,9 @@ __device__ __forceinline__ void potential_gradient_t(const PV &pot, const double
 // The factors of a disk-bulge-halo composite's gradient in gala's expressions, in
 // one straight run (see fast::dbh_gradient): spheres f1, f2, disk fd with mz on
 // its z component, halo fn; s0, s1, s2 are the squares of the coordinates.  False
-// where an argument is outside the integer forms' range.  The bits are those of
-// comp_gradient; side by side the chains take 16,384 uneven FP64 orbits from 35.5
-// to 22.0 ms.
+// where an argument is outside the integer forms' range (the second sphere's G m is
+// +0 or inside it: pack_dbh in gx_host.cu).  The bits are those of comp_gradient; side
+// by side the chains take 16,384 uneven FP64 orbits from 35.5 to 22.0 ms.
 template <bool LIBLN>
 __device__ __forceinline__ bool dbh_factors(const DevPot &pot, double s0, double s1, double s2, double &f1, double &f2,
                                             double &fd, double &mz, double &fn) {

@@ -122,6 +122,11 @@ static void pack_dbh(DevPot *out) {
     }
     out->dbh = (nh == 1 || nh == 2) && nd == 1 && nn == 1;
     if (!out->dbh || out->c[out->ncomp - 1].type != GX_POT_SPHERICALNFW) return;
+    // dbh_factors and gradient_axis take a second sphere's G m of +0 for a missing
+    // sphere and dbh_factors divides any other unchecked: it has to be in the integer
+    // quotient's range (ip::mid_range), else the general form serves the composite
+    const double gm2 = std::fabs(out->d.gm2);
+    if (!(out->d.gm2 == 0. ? !std::signbit(out->d.gm2) : gm2 >= std::ldexp(1.0, -511) && gm2 < std::ldexp(1.0, 511))) return;
     if (out->c[0].type == GX_POT_MIYAMOTONAGAI) out->dbh_order = 2;
     if (out->c[out->ncomp - 2].type == GX_POT_MIYAMOTONAGAI) out->dbh_order = 1;
 }
