@@ -165,6 +165,7 @@ dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ DevFra
         // the CTA is stepping any more
         if (!__syncthreads_or(done ? 0 : 1)) break;
         bool stepping = !done;
+        if (stepping && h != h) nan_steps(nmax, naccpt, nstep, nfcn, nrejct);
         if (stepping && nstep > nmax) {
             idid = -2;
             done = true;
@@ -562,6 +563,7 @@ dop853_static_kernel(const __grid_constant__ DevPot pot, DopArgs A, int G, const
 
     // every scalar below is the same in all warps of the batch
     for (;;) {
+        if (h != h) nan_steps(nmax, naccpt, nstep, nfcn, nrejct);
         if (nstep > nmax) {
             idid = -2;
             break;

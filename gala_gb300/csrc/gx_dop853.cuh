@@ -25,6 +25,17 @@ __device__ __forceinline__ double max_abs(double a, double b) {
     return __longlong_as_double(x > y ? x : y);
 }
 
+// The counters after a NaN step size: no later step is accepted, so gala evaluates
+// eleven stages and rejects, up to nmax + 1 steps, and returns -2 (the state and the
+// stored rows stay as they are).  A batch ends at once with what that comes to; the
+// steps themselves are 1e6 by default, about a minute that no cancellation reaches.
+__device__ __forceinline__ void nan_steps(int64_t nmax, int64_t naccpt, int64_t &nstep, int64_t &nfcn, int64_t &nrejct) {
+    const int64_t left = nmax + 1 - nstep;
+    nstep += left;
+    nfcn += 11 * left;
+    if (naccpt >= 1) nrejct += left;
+}
+
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

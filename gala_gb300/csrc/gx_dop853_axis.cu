@@ -284,6 +284,7 @@ dop853_axis_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ D
 
     // every scalar below is the same in all warps of the batch
     for (;;) {
+        if (h != h) nan_steps(nmax, naccpt, nstep, nfcn, nrejct);
         if (nstep > nmax) {
             idid = -2;
             break;
