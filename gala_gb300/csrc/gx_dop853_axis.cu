@@ -228,8 +228,10 @@ dop853_axis_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ D
     const bool active = j < nb && c < 3;  // a coordinate of an orbit of the batch
     const double nsys = 6 * nb;
 
-    // lanes without an orbit go along at a harmless point and add nothing to the sums
-    double x = j < nb ? w0[axis * n + i0 + j] : 1., v = j < nb ? w0[(3 + axis) * n + i0 + j] : 0.;
+    // lanes without an orbit go along with the batch's last one and add nothing to the sums: an
+    // orbit of their own would choose between the forms of the force for the real ones in its warp
+    const int jw = min(j, nb - 1);
+    double x = w0[axis * n + i0 + jw], v = w0[(3 + axis) * n + i0 + jw];
     double x1, x2, x3, x4, x5, x6, x7, x8, x9, x10, v1, v2, v3, v4, v5, v6, v7, v8, v9, v10, xs, vs, xn, vn;
 
     // dop853() front-end defaults with dop853_helper's arguments (dop853.pyx:157-182)
