@@ -141,6 +141,7 @@ SIGNATURES = {
     "gx_stream_sample": (C.c_int, [_PP, _I64, _I64, _P, _I64, _P, _P, _P, _I64, _I32, _P, _D, _I32, _I32, _I32, _P,
                                    _P]),
     "gx_batch_integrate_fp64": (C.c_int, [_PP, _P, _I64, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P, _P]),
+    "gx_batch_fp64_lanes": (C.c_int, [_PP, _I64, _P]),
     "gx_batch_schedule_slots": (C.c_int64, [_I64, _I32]),
     "gx_batch_schedule_work_words": (C.c_int64, [_I64, _I32]),
     "gx_batch_schedule": (C.c_int, [_P, _P, _I64, _I32, _P, _I64, _P, _I64, _P]),

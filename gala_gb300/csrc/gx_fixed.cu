@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(128, 1) batch_fp64_kernel(const __grid_constan
 
 // The batch with four lanes per orbit: a CTA of four warps takes a 32-orbit block,
 // eight orbits to a warp, one CTA per SM.  For batches whose longest orbits set the
-// time rather than the FP64 pipe's throughput (few_batch_orbits): lengths 100 to
+// time rather than the FP64 pipe's throughput (batch_lanes): lengths 100 to
 // 2,000, MW composite, 16,384 orbits 22.0 ms one lane per orbit, 11.9 ms here; 24,000
 // 22.0 and 12.8; 40,001 22.0 and 21.2.  (Four such CTAs per SM: 25.5 ms for 16,384,
 // the longest orbits then share their scheduler from the start.)
@@ -402,10 +402,24 @@ __global__ void __launch_bounds__(128) batch_axis_kernel(const __grid_constant__
     }
 }
 
-// Whether a batch is small enough for four lanes per orbit: 160 orbits per SM, where
-// the two forms meet for lengths spread 5 : 1 (26,000 orbits; for 20 : 1 it is 41,000).
-static bool few_batch_orbits(const DevPot &dp, int64_t n) {
-    return !dp.has_scf && !dp.cdev && n <= (int64_t)160 * multiprocessors();
+// Lanes per orbit of a batch.  An SM takes 32 orbits at a time with four lanes each, and
+// one after another beyond that, while one lane per orbit takes 128 at a time: what the
+// four lanes gain is a shorter step, and the lengths decide what that is worth.  300
+// steps on average, one lane / four, ms:
+//   straight run of a composite (0.55 of the step): even Ruth4 lengths 4,864 orbits 3.36
+//   / 1.84, 9,800 3.36 / 5.38; spread 20 : 1 17,000 6.61 / 3.59, 24,320 6.60 / 3.92.  The
+//   line is where spread lengths still gain (5 : 1 meets there, 20 : 1 at 41,000).
+//   one Hernquist sphere (0.45): even Ruth4 9,728 1.86 / 1.61, 14,700 1.86 / 3.12, even
+//   Leapfrog 9,728 0.59 / 0.51, 9,800 0.59 / 0.74; 20 : 1 17,000 3.62 / 1.59.  With steps
+//   that cheap even lengths are to gain too.
+//   component loop (0.83 to 0.9: a lane still evaluates every component): even Ruth4, five
+//   to eight components 4,864 0.9, 5,000 1.7 times one lane's; 20 : 1 24,320 0.97.  One
+//   block per SM.
+static int batch_lanes(const DevPot &dp, int64_t n) {
+    if (dp.has_scf || dp.cdev) return 1;
+    const int mode = axis_mode(dp);
+    const int64_t per_sm = mode == 0 ? 32 : mode == 1 ? 64 : 160;
+    return n <= per_sm * multiprocessors() ? 4 : 1;
 }
 
 static int fixed_common(const gx_potential *pot, const gx_frame *frame, const double *w0, int64_t n,
@@ -475,7 +489,7 @@ int gx_batch_integrate_fp64(const gx_potential *pot, const double *w0, int64_t n
     cudaStream_t st = gx::as_stream(stream);
     GX_CUDA_TRY(cudaMemsetAsync(queue_counter, 0, GX_BATCH_QUEUE_WORDS * sizeof(int32_t), st));
     const int64_t n_lead = gx::queue_lead_chunks(n_slots / chunk, chunk);
-    if (gx::few_batch_orbits(dp, n)) {
+    if (gx::batch_lanes(dp, n) == 4) {
         const auto kernel = gx::axis_mode(dp) == 0   ? gx::batch_axis_kernel<0>
                             : gx::axis_mode(dp) == 1 ? gx::batch_axis_kernel<1>
                             : gx::axis_mode(dp) == 2 ? gx::batch_axis_kernel<2>
@@ -492,6 +506,16 @@ int gx_batch_integrate_fp64(const gx_potential *pot, const double *w0, int64_t n
         gx::batch_fp64_kernel<false><<<grid, block, 0, st>>>(dp, co, n, n_slots, chunk, n_lead, w0, n_steps, dt,
                                                              method, order, queue_counter, w_out, gx::cancel_flag());
     return gx::check_launch("batch_fp64");
+}
+
+int gx_batch_fp64_lanes(const gx_potential *pot, int64_t n, int32_t *lanes) {
+    gx::DevPot dp;
+    int rc = gx::pack_potential(pot, &dp);
+    if (rc) return rc;
+    GX_CHECK_ARG(n >= 0, "n < 0");
+    GX_CHECK_ARG(lanes, "NULL pointer");
+    *lanes = gx::batch_lanes(dp, n);
+    return GX_OK;
 }
 
 int gx_ruth4_integrate_hamiltonian(const gx_potential *pot, const gx_frame *frame, const double *w0, int64_t n,

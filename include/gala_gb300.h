@@ -384,12 +384,18 @@ int gx_batch_integrate_fp32_state(const gx_potential* pot, const double* w0, int
 /* The plain FP64 form of the same batched workload: identical arguments and
  * queue; per orbit, gala's Leapfrog / Ruth4 arithmetic in FP64 exactly as
  * gx_leapfrog_integrate_hamiltonian / gx_ruth4_integrate_hamiltonian compute it
- * (bit-identical final states).  block <= 128.  SCF components allowed. */
+ * (bit-identical final states).  block <= 128.  SCF components allowed.  Batches of
+ * few orbits take four lanes per orbit (gx_batch_fp64_lanes), always in CTAs of 128
+ * threads and at most one per multiprocessor. */
 int gx_batch_integrate_fp64(const gx_potential* pot, const double* w0, int64_t n,
                             const int64_t* n_steps, const double* dt, const int32_t* method,
                             const int32_t* order, int64_t n_slots, int32_t chunk,
                             int32_t block, int32_t grid, int32_t* queue_counter,
                             double* w_out, void* stream);
+
+/* How many lanes of a warp gx_batch_integrate_fp64 gives each of n orbits on the
+ * current device (HOST int32 *lanes): 4 or 1.  No counterpart in gala. */
+int gx_batch_fp64_lanes(const gx_potential* pot, int64_t n, int32_t* lanes);
 
 /* Allocation-free form of gx_batch_integrate_fp32.  No counterpart in gala.
  * For callers that cannot allocate device memory (a process whose memory
