@@ -145,6 +145,7 @@ SIGNATURES = {
     "gx_batch_schedule_slots": (C.c_int64, [_I64, _I32]),
     "gx_batch_schedule_work_words": (C.c_int64, [_I64, _I32]),
     "gx_batch_schedule": (C.c_int, [_P, _P, _I64, _I32, _P, _I64, _P, _I64, _P]),
+    "gx_dop853_form": (C.c_int, [_PP, _PF, _I64, _I32, _P]),
     "gx_dop853_integrate_hamiltonian": (
         C.c_int,
         [_PP, _PF, _P, _I64, _P, _I64, _D, _D, _I64, _D, _I64, _I32, _I32, _I64, _P, _P, _P, _P],

@@ -865,7 +865,37 @@ static cudaError_t launch_static(const DevPot &dp, const DopArgs &A, int G, cons
                       : cudaLaunchKernelEx(&cfg, dop853_static_kernel<false>, dp, A, G, w0, n, t, out, status, stats);
 }
 
+// The kernel that takes a call.
+static int dop853_form(const DevPot &dp, const DevFrame &df, const DopArgs &A, int64_t n) {
+    // Few orbits: one coordinate per lane.
+    if (dop853_axis_takes(dp, df, A, n)) return GX_DOP853_AXIS;
+    // A static frame and a batch that fills one to eight warps (the portable cluster
+    // size): a cluster per batch.  Several batches of at most 16 orbits stay with the general
+    // kernel, where two of them share a warp and with it each FP64 instruction.
+    const int64_t nbatches = (n + A.nbatch - 1) / A.nbatch;
+    const int64_t G = ((A.nbatch < n ? A.nbatch : n) + 31) / 32;
+    if (df.type == GX_FRAME_STATIC && G <= NYS_MAX_WARPS && (A.nbatch > 16 || nbatches == 1) && nbatches * G < ((int64_t)1 << 31))
+        return GX_DOP853_CLUSTER;
+    return GX_DOP853_GENERAL;
+}
+
 }  // namespace gx
+
+extern "C" int gx_dop853_form(const gx_potential *pot, const gx_frame *frame, int64_t n, int32_t nbatch, int32_t *form) {
+    gx::DevPot dp;
+    gx::DevFrame df;
+    int rc = gx::pack_potential(pot, &dp);
+    if (rc) return rc;
+    rc = gx::pack_frame(frame, &df);
+    if (rc) return rc;
+    GX_CHECK_ARG(n >= 0, "n < 0");
+    GX_CHECK_ARG(nbatch >= 1 && nbatch <= 1024, "nbatch must be in [1, 1024] (got %d)", nbatch);
+    GX_CHECK_ARG(form, "NULL pointer");
+    gx::DopArgs A = {};
+    A.nbatch = nbatch;
+    *form = gx::dop853_form(dp, df, A, n);
+    return GX_OK;
+}
 
 extern "C" int gx_dop853_integrate_hamiltonian(const gx_potential *pot, const gx_frame *frame, const double *w0,
                                                int64_t n, const double *t, int64_t ntimes, double atol,
@@ -901,15 +931,10 @@ extern "C" int gx_dop853_integrate_hamiltonian(const gx_potential *pot, const gx
     A.nbatch = nbatch;
     const int64_t nbatches = (n + nbatch - 1) / nbatch;
     cudaStream_t st = gx::as_stream(stream);
-    // Few orbits: one coordinate per lane.
-    if (gx::dop853_axis_takes(dp, df, A, n)) return gx::launch_dop853_axis(dp, df, A, w0, n, t, w_out, status, stats, st);
-    // A static frame and a batch that fills one to eight warps (the portable cluster
-    // size): a cluster per batch.  Several batches of at most 16 orbits stay below,
-    // where two of them share a warp and with it each FP64 instruction.
-    const int64_t per = nbatch < n ? nbatch : n;
-    const int G = (int)((per + 31) / 32);
-    if (df.type == GX_FRAME_STATIC && G <= gx::NYS_MAX_WARPS && (nbatch > 16 || nbatches == 1) &&
-        nbatches * G < ((int64_t)1 << 31)) {
+    const int form = gx::dop853_form(dp, df, A, n);
+    if (form == GX_DOP853_AXIS) return gx::launch_dop853_axis(dp, df, A, w0, n, t, w_out, status, stats, st);
+    if (form == GX_DOP853_CLUSTER) {
+        const int G = (int)(((nbatch < n ? nbatch : n) + 31) / 32);
         const cudaError_t e = gx::launch_static(dp, A, G, w0, n, t, w_out, status, stats, st);
         if (e != cudaSuccess) {
             gx::set_error("dop853 launch failed: %s", cudaGetErrorString(e));

@@ -288,6 +288,15 @@ int gx_dop853_integrate_hamiltonian(const gx_potential* pot, const gx_frame* fra
                                     int64_t out_stride, double* w_out,
                                     int32_t* status, int64_t* stats, void* stream);
 
+/* The kernel that gx_dop853_integrate_hamiltonian takes for n orbits in batches of
+ * nbatch on the current device (HOST int32 *form).  No counterpart in gala. */
+typedef enum gx_dop853_kernel {
+    GX_DOP853_GENERAL = 0,  /* one CTA per batch or two; any frame              */
+    GX_DOP853_CLUSTER = 1,  /* a cluster of one-warp CTAs per batch, static     */
+    GX_DOP853_AXIS = 2      /* one coordinate per lane, few orbits              */
+} gx_dop853_kernel;
+int gx_dop853_form(const gx_potential* pot, const gx_frame* frame, int64_t n, int32_t nbatch, int32_t* form);
+
 /* FP32-compensated form of leapfrog_integrate_hamiltonian / ruth4_integrate_
  * hamiltonian (src/gala/integrate/cyintegrators/leapfrog.pyx:54-121,
  * ruth4.pyx:37-113) on gala's time grid (step t[1] - t[0]): FP32 forces,
