@@ -561,10 +561,9 @@ class Orbit(PhaseSpacePosition):
         _abi.call("gx_orbit_extrema", ptr(wd), ptr(td), nt, n, int(bool(approximate)), int(keep), ptr(count),
                   ptr(sm), ptr(mn), ptr(mx), ptr(vals) if keep else None, ptr(times) if keep else None,
                   stream_handle())
-        host = torch.empty(stats.shape, dtype=stats.dtype, pin_memory=True)
-        host.copy_(stats, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        host = host.numpy()
+        # into ordinary memory, which the orbit keeps: through a page-locked block, kept or copied
+        # out of, 20,011 orbits took 58 and 178 us for 51
+        host = stats.cpu().numpy()
         out = {k: host[3 * n * i:3 * n * (i + 1)].reshape(3, n) for i, k in enumerate(("sum", "min", "max"))}
         out["count"] = host[9 * n:].view(np.int32)[:3 * n].reshape(3, n)
         if keep:
