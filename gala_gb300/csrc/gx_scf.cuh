@@ -26,7 +26,9 @@
 // 3,800 FP64 instructions at nmax = 12, lmax = 8.  131,101 points, potential and
 // gradient, to host arrays: 1.8 ms (34.4 ms when each term formed its own norm,
 // powers and quotients).  As in gala a term whose S and T are both zero is left
-// out, so that a non-finite factor (on the pole, say) does not reach it.
+// out, so that a non-finite factor (on the pole, say) does not reach it, and at the
+// centre, where every term of the density is infinite, they are summed one by one:
+// terms of both signs make it NaN.
 #pragma once
 
 #include "gx_device.cuh"
@@ -36,6 +38,24 @@ namespace gx {
 
 constexpr int SCF_MAX_N = 24;   // nmax + 1
 constexpr int SCF_MAX_L = 16;   // lmax + 1
+
+// The density where s is 0: gala's sum of its terms there, each infinite for l = 0
+// (C_n^{3/2}(-1) alternates in sign) and 0 / 0 for the others, so infinite only where
+// every term has one sign.
+static __device__ __noinline__ double scf_density_centre(const double *p, int nmax, int lmax) {
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    const int sn = (lmax + 1) * (lmax + 1);
+    double acc = 0.;
+    for (int n = 0; n <= nmax; n++)
+        for (int l = 0; l <= lmax; l++)
+            for (int m = 0; m <= l; m++) {
+                const int i = 5 + n * sn + m + (lmax + 1) * l;
+                const double S = p[i], T = p[i + (nmax + 1) * sn];
+                if (S == 0. && T == 0.) continue;
+                acc += l == 0 ? (S + 0. * T) * (n & 1 ? -inf : inf) : inf - inf;
+            }
+    return acc * p[3];
+}
 
 // kind 0: value, 1: gradient (accumulated into g), 2: density.
 template <int KIND>
@@ -56,8 +76,17 @@ __device__ __forceinline__ double scf_eval(const double *p, const double *q, dou
     const double X = q[2] * ir, st = R * ir;
     const double i1 = ddiv(1.0, s1);
     const double xi = (s - 1.0) * i1;
-    const double iR = R2 == 0. ? 0. : ddiv(1.0, R);
-    const double cp = R2 == 0. ? 1. : q[0] * iR, sp = q[1] * iR;  // atan2(0, 0) = 0
+    double cp, sp;
+    if (R2 > 0x1p-900) {
+        const double iR = ddiv(1.0, R);
+        cp = q[0] * iR;
+        sp = q[1] * iR;
+    } else {  // R2 has lost digits or underflowed: the angle from the coordinates scaled up
+        const double x = q[0] * 0x1p600, y = q[1] * 0x1p600, Rs = sqrt(fma(x, x, y * y));
+        cp = Rs == 0. ? 1. : x / Rs;  // atan2(0, 0) = 0
+        sp = Rs == 0. ? 0. : y / Rs;
+    }
+    if (KIND == 2 && s == 0.) return scf_density_centre(p, nmax, lmax);
 
     double C[SCF_MAX_N], D[SCF_MAX_N];                       // C_n^a, C_{n-1}^{a+1}
     double Pl[SCF_MAX_L], Pl1[SCF_MAX_L], Pl2[SCF_MAX_L];    // P_l^m of this l and the two before
