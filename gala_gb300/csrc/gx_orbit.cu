@@ -401,8 +401,8 @@ __device__ __forceinline__ void ext_store(const ExtArgs &A, int k, int64_t i, in
     A.vmax[k * A.n + i] = count ? from_key(kmax) : nan;
 }
 
-// 16 bytes of partial statistics of another CTA of the cluster: the same shared
-// address in CTA `rank`.
+// The partial statistics of another CTA of the cluster: the same shared address in
+// CTA `rank`.
 __device__ __forceinline__ const ExtPart *ext_remote(const ExtPart *p, unsigned rank) {
     unsigned long long r;
     asm volatile("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
@@ -463,14 +463,20 @@ __global__ void __launch_bounds__(EXT_THREADS, 2) orbit_extrema_kernel(const Ext
                 int32_t count = 0;
                 double sum = 0.;
                 long long kmin = 0x7fffffffffffffffLL, kmax = -0x7fffffffffffffffLL - 1;
-                for (int w = 0; w < segs; w++) {
-                    const ExtPart *Q = reinterpret_cast<const ExtPart *>(&warps[w % EXT_WARPS].rings.r[0][0]);
-                    if (w >= EXT_WARPS) Q = ext_remote(Q, w / EXT_WARPS);
-                    if (Q->count[k][lane] == 0) continue;
-                    count += Q->count[k][lane];
-                    sum += Q->sum[k][lane];
-                    kmin = min(kmin, Q->kmin[k][lane]);
-                    kmax = max(kmax, Q->kmax[k][lane]);
+                // a CTA's segments first, then the CTAs' sums: with one sum over all segments its
+                // rounding grows with the cluster (a segment of 64 holds an extremum or two)
+                for (int r = 0; r < cluster; r++) {
+                    double part = 0.;
+                    for (int w = 0; w < EXT_WARPS; w++) {
+                        const ExtPart *Q = reinterpret_cast<const ExtPart *>(&warps[w].rings.r[0][0]);
+                        if (r > 0) Q = ext_remote(Q, r);
+                        if (Q->count[k][lane] == 0) continue;
+                        count += Q->count[k][lane];
+                        part += Q->sum[k][lane];
+                        kmin = min(kmin, Q->kmin[k][lane]);
+                        kmax = max(kmax, Q->kmax[k][lane]);
+                    }
+                    sum += part;
                 }
                 if (io < A.n) ext_store(A, k, io, count, sum, kmin, kmax);
             }
