@@ -306,8 +306,25 @@ class BatchIntegrator:
         except KeyError:
             return dict(DEFAULT_CONFIG[self.precision])
 
+    def _launch_shapes(self):
+        """The launch shapes that differ for this batch: SEARCH, or, for an FP64 batch
+        with four lanes per orbit (always one CTA of 128 threads per multiprocessor),
+        SEARCH's chunk sizes with the block and CTA count of the record in use.  Noise
+        between equal launches would else choose the shape of larger batches, which
+        share the record."""
+        import ctypes as C
+
+        shapes = SEARCH[self.precision]
+        if self.precision == "fp64":
+            lanes = C.c_int32()
+            _abi.call("gx_batch_fp64_lanes", self.potential.packed().for_device(), self.n, C.addressof(lanes))
+            if lanes.value == 4:
+                base = self._cached_config()
+                shapes = [{**base, "chunk": k} for k in sorted({c["chunk"] for c in shapes})]
+        return shapes
+
     def autotune(self, work_fraction=0.03, reps=2, persist=True):
-        """Time every launch shape of SEARCH on a scaled copy of this workload --
+        """Time the launch shapes of SEARCH on a scaled copy of this workload --
         all orbits, every step count multiplied by `work_fraction` (at least 1),
         so the number of warps and the spread of orbit lengths are those of the
         real run -- keep the fastest and cache it."""
@@ -320,7 +337,7 @@ class BatchIntegrator:
                               config=DEFAULT_CONFIG[self.precision], precision=self.precision)
         results = []
         stream = torch.cuda.current_stream()
-        for cfg in SEARCH[self.precision]:
+        for cfg in self._launch_shapes():
             sub.config = cfg
             sub._launch_integrator(stream_handle())
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

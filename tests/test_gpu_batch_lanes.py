@@ -35,3 +35,29 @@ def test_lines_between_the_forms(name, per_sm):
     w0, ns, m = W.mw_ics(line + 1, seed=3), np.full(line + 1, 4), (np.arange(line + 1) % 2).astype(np.int32)
     a, b = (BatchIntegrator(pot, w0[:, :n], ns[:n], np.full(n, 0.5), m[:n], precision="fp64").run().cpu().numpy() for n in (line, line + 1))
     assert np.array_equal(a, b[:, :line])
+
+
+@pytest.mark.parametrize("extra,shapes", [(0, 2), (1, None)])
+def test_autotune_times_the_shapes_that_differ(tmp_path, monkeypatch, extra, shapes):
+    """Four lanes per orbit ignore block and CTA count: only the chunk is searched, and the
+    record keeps the block and CTA count that larger batches were tuned to."""
+    import json
+
+    import torch
+
+    import gala_gb300.batch as B
+    from gala_gb300 import workloads as W
+
+    cache = tmp_path / "autotune.json"
+    monkeypatch.setattr(B, "CACHE", cache)
+    n = 32 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    args = (_pot("plummer"), W.mw_ics(n, seed=3), np.full(n, 4), np.full(n, 0.5), np.zeros(n, dtype=np.int32))
+    key = B.BatchIntegrator(*args, precision="fp64")._cache_key()
+    tuned = {"block": 64, "ctas_per_sm": 8, "chunk": 64}
+    cache.write_text(json.dumps({key: tuned}))
+    b = B.BatchIntegrator(*args, precision="fp64")
+    best = b.autotune(work_fraction=1.0, reps=1)
+    record = json.loads(cache.read_text())[key]
+    assert record == best and len(b.tune_results) == (shapes or len(B.SEARCH["fp64"]))
+    if shapes:
+        assert {k: best[k] for k in ("block", "ctas_per_sm")} == {k: tuned[k] for k in ("block", "ctas_per_sm")}
