@@ -262,13 +262,6 @@ static int launch_axis(const DevPot &dp, const Ruth4Coef &co, const double *w0, 
     return check_launch(name);
 }
 
-static int multiprocessors() {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 0;
-    return sms;
-}
-
 // Whether few enough orbits for one coordinate per lane.
 static bool few_orbits(const DevPot &dp, int64_t n) { return !dp.has_scf && !dp.cdev && n <= (int64_t)32 * multiprocessors(); }
 

@@ -55,6 +55,14 @@ __device__ __forceinline__ bool cancel_requested(const int32_t *flag) {
     return flag != nullptr && *reinterpret_cast<const volatile int32_t *>(flag) != 0;
 }
 
+// Multiprocessors of the current device (0 without one).
+inline int multiprocessors() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return sms;
+}
+
 // Launch-error check after a <<<>>> launch.
 inline int check_launch(const char *what) {
     cudaError_t e = cudaGetLastError();

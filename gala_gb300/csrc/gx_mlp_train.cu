@@ -19,6 +19,7 @@
 // that follows it in its epilogue; grads_kernel for the weights); the products with the
 // 3-wide input or gradient are row and column reductions of their own.  What bounds a
 // step is the FP32 pipe: 18 products of batch x 256 x 256.  Batch 8,192, 16 steps: 21.1 -> 12.5 ms.
+#include <algorithm>
 #include <cooperative_groups.h>
 
 #include "gx_host.h"
@@ -337,7 +338,8 @@ static void rows(cudaStream_t st, int64_t batch, const float *A, const float *W,
 // C += A^T B over the batch
 static void weight_grads(cudaStream_t st, int64_t batch, const float *A, const float *B, float *C) {
     constexpr int TILES = (H / BM) * (H / BN);
-    const int64_t split = 2 * 152 / TILES;
+    // whole pairs of CTAs, no more than two CTAs on every SM: a pair beyond is a second wave
+    const int64_t split = std::max(2 * gx::multiprocessors() / TILES / 2 * 2, 2);
     const int share = (int)(((batch + split - 1) / split + BK - 1) / BK * BK);
     const dim3 grid(H / BN, H / BM, (nblk(batch, share) + 1) / 2 * 2);
     if (aligned16(A, B, C))
