@@ -57,7 +57,7 @@ struct DevPot {
                           // GX_MAX_COMPONENTS components), else null
     int32_t dbh;          // a disk-bulge-halo composite: see d
     int32_t dbh_order;    // and its order: 1 spheres, disk, halo; 2 disk, spheres, halo; 0 another
-    int32_t sphere;       // one unshifted Hernquist or Plummer sphere: its type (d.gm1; d.c1 = c or b^2), else 0
+    int32_t sphere;       // GX_POT_HERNQUIST for one unshifted Hernquist sphere (d.gm1, d.c1), else 0
     int32_t pad;
     DevComp c[GX_MAX_COMPONENTS];
     double p[GX_MAX_INLINE_PARAMS];
@@ -152,7 +152,7 @@ struct Radius {
 // Whether the gradient at x is finite for certain, so that gala's product of it
 // with a zero coefficient (the first sub-step of Ruth4) is zero: `regular` says
 // that every component is a closed form centred on the origin with parameters of
-// ordinary size (regular_potential in gx_host.cu), and the largest coordinate
+// ordinary size (regular_component in gx_host.cu), and the largest coordinate
 // lies within 2^-100 and 2^100.
 __device__ __forceinline__ bool ordinary(double v) {
     return ((unsigned)__double2hiint(v) & 0x7fffffffu) - (923u << 20) < (200u << 20);

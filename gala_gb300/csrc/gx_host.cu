@@ -64,7 +64,9 @@ static void derived_constants(int type, const double *P, DevComp &d) {
 // within 2^-100 and 2^100: centred on the origin, every length positive (Hernquist
 // c and Miyamoto-Nagai a may be 0, Plummer b anything) and every parameter of
 // ordinary size.  Then no intermediate of its gradient leaves the FP64 range (the
-// largest is G m / r_s / u^3 / r_s^2 with u = r / r_s >= 2^-160) and no divisor is zero.
+// largest is G m / r_s / u^3 / r_s^2 with u the radius, scaled by the axes, over r_s:
+// u >= 2^-100 / 2^60 / 2^60 = 2^-220, so below 2^(180 + 660 + 120); and u <= 2^221) and
+// no divisor is zero.
 static bool regular_component(int type, const double *P, int do_sr) {
     if (do_sr) return false;
     auto small = [](double v) { return std::fabs(v) <= std::ldexp(1.0, 60); };
@@ -84,14 +86,13 @@ static bool regular_component(int type, const double *P, int do_sr) {
     }
 }
 
-// Whether the packed components are a single sphere or a disk-bulge-halo composite;
-// its constants.
+// Whether the packed components are a single Hernquist sphere or a disk-bulge-halo
+// composite; its constants.
 static void pack_dbh(DevPot *out) {
-    if (out->ncomp == 1 && !out->c[0].do_sr &&
-        (out->c[0].type == GX_POT_HERNQUIST || out->c[0].type == GX_POT_PLUMMER)) {
-        out->sphere = out->c[0].type;
+    if (out->ncomp == 1 && !out->c[0].do_sr && out->c[0].type == GX_POT_HERNQUIST) {
+        out->sphere = GX_POT_HERNQUIST;
         out->d.gm1 = out->c[0].dc[0];
-        out->d.c1 = out->c[0].type == GX_POT_PLUMMER ? out->c[0].dc[1] : out->p[out->c[0].poff + 2];
+        out->d.c1 = out->p[out->c[0].poff + 2];
         return;
     }
     out->d.gm2 = 0.;
