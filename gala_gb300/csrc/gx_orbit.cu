@@ -464,13 +464,14 @@ __global__ void __launch_bounds__(EXT_THREADS, 2) orbit_extrema_kernel(const Ext
                 double sum = 0.;
                 long long kmin = 0x7fffffffffffffffLL, kmax = -0x7fffffffffffffffLL - 1;
                 // a CTA's segments first, then the CTAs' sums: with one sum over all segments its
-                // rounding grows with the cluster (a segment of 64 holds an extremum or two)
+                // rounding grows with the cluster (a segment of 64 holds an extremum or two).  A
+                // segment without any is neutral in all four, so no load waits on a count.
                 for (int r = 0; r < cluster; r++) {
                     double part = 0.;
+#pragma unroll
                     for (int w = 0; w < EXT_WARPS; w++) {
                         const ExtPart *Q = reinterpret_cast<const ExtPart *>(&warps[w].rings.r[0][0]);
                         if (r > 0) Q = ext_remote(Q, r);
-                        if (Q->count[k][lane] == 0) continue;
                         count += Q->count[k][lane];
                         part += Q->sum[k][lane];
                         kmin = min(kmin, Q->kmin[k][lane]);
