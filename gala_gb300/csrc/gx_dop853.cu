@@ -673,7 +673,9 @@ dop853_static_kernel(const __grid_constant__ DevPot pot, DopArgs A, int G, const
         nys_sum2(err, err2, buf[par], G, rank);
         par ^= 1;
         double deno = fma(0.01, err2, err);
-        if (deno <= 0.0) deno = 1.0;
+        // gala's deno <= 0, and where its reciprocal would overflow: the estimates hold nothing but
+        // accelerations (no rounding of the velocities), so nearly free orbits come that low
+        if (deno < 0x1p-1000) deno = 1.0;
         err = fabs(h) * err * dsqrt(ddiv(1.0, deno * nsys));
         // computation of hnew (:446-452); gala's pow(err, 1/8) (beta = 0) as three square roots
         const double fac11 = dsqrt(dsqrt(dsqrt(err)));
