@@ -418,7 +418,7 @@ dop853_kernel(const __grid_constant__ DevPot pot, const __grid_constant__ DevFra
 // CTA of the cluster, one cluster barrier, and all add the partial sums in rank
 // order, so all take the same decisions.
 //
-// Measured: 20,011 MW orbits x 1 Gyr (201 batches) 180 -> 84 ms (230 ms before the
+// Measured: 20,011 MW orbits x 1 Gyr (201 batches) 180 -> 86 ms (230 ms before the
 // force left the FP64 pipe), now 823 FP64 instructions per step and warp and bound
 // by the FP64 units of the SMs that hold six warps.
 // ---------------------------------------------------------------------------

@@ -6,7 +6,7 @@
 // cycles whatever its lanes do, and a few batches of orbits leave most of the 608
 // schedulers idle, so the coordinates go side by side: a step takes about 500
 // FP64 instructions instead of 823 (static frame) or 1,500 (rotating frame).  37
-// orbits through a rotating bar, 400 Myr, every Myr kept: 54 -> 15 ms.
+// orbits through a rotating bar, 400 Myr, every Myr kept: 59 -> 18 ms (one lane per orbit / here).
 //   * A batch is a cluster of up to 8 CTAs of 1, 2 or 4 warps, 8 orbits to a warp
 //     (100 orbits: 7 CTAs of 2 warps), spread over as many SMs.
 //   * The right-hand side gathers the point by shuffles, and each lane evaluates one of

@@ -212,7 +212,7 @@ __device__ __forceinline__ void potential_gradient_ft(const PV &pot, const doubl
 // instructions, and the two square roots, the inverse root, the three reciprocals
 // and the logarithm on the integer pipe side by side instead of one after the
 // other behind the component loop's branches (with it the DOP853 population of 20,011
-// orbits x 1 Gyr takes 84 ms, without 134).  False where an argument is outside the integer forms' range (a point
+// orbits x 1 Gyr takes 86 ms, without 134).  False where an argument is outside the integer forms' range (a point
 // within 2^-6 r_s of the centre, a non-finite position): the general form then
 // serves.
 __device__ __forceinline__ bool dbh_gradient(const DevPot &pot, const double *q, double *g) {

@@ -17,8 +17,11 @@
 // Parameter gradients are written to `grads`; gx_mlp_adam applies Adam.
 // Every 256-wide product is a tiled FP32 kernel (rows_kernel, with the elementwise pass
 // that follows it in its epilogue; grads_kernel for the weights); the products with the
-// 3-wide input or gradient are row and column reductions of their own.  What bounds a
-// step is the FP32 pipe: 18 products of batch x 256 x 256.  Batch 8,192, 16 steps: 21.1 -> 12.5 ms.
+// 3-wide input or gradient are row and column reductions of their own.  Most of a step is
+// 18 products of batch x 256 x 256 at about half the rate of the FP32 pipe: two 128 x 64
+// tiles on an SM (84 % of the slots at batch 8,192) that wait for their slabs and for one
+// another, and the start and end of each of 42 launches.  Batch 8,192, 16 steps: 21.1 ->
+// 12.6 ms.
 #include <algorithm>
 #include <cooperative_groups.h>
 

@@ -24,7 +24,7 @@
 //   sin theta = R / r (gala's sqrt(1 - X^2) loses digits near the pole).
 // What bounds it is the FP64 pipe: per gradient 4 multiply-adds per (n, l, m), about
 // 3,800 FP64 instructions at nmax = 12, lmax = 8.  131,101 points, potential and
-// gradient, to host arrays: 1.8 ms (34.4 ms when each term formed its own norm,
+// gradient, to host arrays: 1.5 ms (34.4 ms when each term formed its own norm,
 // powers and quotients).  As in gala a term whose S and T are both zero is left
 // out, so that a non-finite factor (on the pole, say) does not reach it, and at the
 // centre, where every term of the density is infinite, they are summed one by one:
